@@ -372,27 +372,37 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
         AQ_CUDA(launch_gather<3>(x->fast, x->consts, a, s));
     else
         AQ_CUDA(launch_gather<2>(x->fast, x->consts, a, s));
-    if (x->consts.boundary == AQUA_BOUNDARY_BI) {
+    // the quad sweep: BI walls, and wherever a clustered choice (the default)
+    // is set but the clustered sweep does not apply
+    const bool bi = x->consts.boundary == AQUA_BOUNDARY_BI;
+    const bool quad = !clustered && (bi || x->sweep_variant >= kSweepClustered);
+    if (quad) {
         if (x->dims == 3)
-            AQ_CUDA(launch_bi_walls<3>(x->fast, x->consts, a, s));
+            AQ_CUDA(launch_clusters<3>(x->consts, a, s));
         else
-            AQ_CUDA(launch_bi_walls<2>(x->fast, x->consts, a, s));
+            AQ_CUDA(launch_clusters<2>(x->consts, a, s));
+    }
+    if (bi) {
+        if (x->dims == 3)
+            AQ_CUDA(launch_bi_walls<3>(x->fast, x->consts, a, (unsigned)x->sms, s));
+        else
+            AQ_CUDA(launch_bi_walls<2>(x->fast, x->consts, a, (unsigned)x->sms, s));
     }
     if (x->profiling)
         AQ_CUDA(cudaEventRecordWithFlags(x->ev[2], s, cudaEventRecordExternal));
     if (clustered) {
         AQ_CUDA(fast::launch_sweep_cl(cst, a, x->sweep_grid, x->sweep_variant,
                                       (unsigned)x->sms, s));
-    } else {
-        // a clustered choice where the clustered sweep does not apply falls
-        // back to the direct sweep's untuned shape
-        const bool cl_pick = x->sweep_variant >= kSweepClustered;
-        const int v = cl_pick ? 9 : x->sweep_variant;
-        const unsigned g = cl_pick ? (unsigned)x->sms * 14u : x->sweep_grid;
+    } else if (quad) {
         if (x->dims == 3)
-            AQ_CUDA(launch_sweep<3>(x->fast, cst, a, g, v, s));
+            AQ_CUDA(launch_sweep_quad<3>(x->fast, cst, a, (unsigned)x->sms, s));
         else
-            AQ_CUDA(launch_sweep<2>(x->fast, cst, a, g, v, s));
+            AQ_CUDA(launch_sweep_quad<2>(x->fast, cst, a, (unsigned)x->sms, s));
+    } else {
+        if (x->dims == 3)
+            AQ_CUDA(launch_sweep<3>(x->fast, cst, a, x->sweep_grid, x->sweep_variant, s));
+        else
+            AQ_CUDA(launch_sweep<2>(x->fast, cst, a, x->sweep_grid, x->sweep_variant, s));
     }
     if (x->profiling)
         AQ_CUDA(cudaEventRecordWithFlags(x->ev[3], s, cudaEventRecordExternal));

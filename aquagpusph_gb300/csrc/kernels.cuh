@@ -179,11 +179,22 @@ cudaError_t launch_free_surface(int dims, const float* r, const int32_t* imove,
 
 template<int D>
 cudaError_t launch_bi_walls(bool fast, const Consts& c, const StepArgs& a,
-                            cudaStream_t s);
+                            unsigned sms, cudaStream_t s);
+// clusters of at most 8 particles of one cell (clu, cperm) and the sweep
+// over them
+template<int D>
+cudaError_t launch_clusters(const Consts& c, const StepArgs& a, cudaStream_t s);
+template<int D>
+cudaError_t launch_sweep_quad(bool fast, const Consts& c, const StepArgs& a,
+                              unsigned sms, cudaStream_t s);
 
 namespace exact {
 template<int D>
-cudaError_t launch_bi_walls_impl(const Consts& c, const StepArgs& a, cudaStream_t s);
+cudaError_t launch_bi_walls_impl(const Consts& c, const StepArgs& a, unsigned sms,
+                                 cudaStream_t s);
+template<int D>
+cudaError_t launch_sweep_quad_impl(const Consts& c, const StepArgs& a,
+                                   unsigned sms, cudaStream_t s);
 template<int D>
 cudaError_t launch_gather_impl(const Consts& c, const StepArgs& a, cudaStream_t s);
 template<int D>
@@ -197,7 +208,11 @@ cudaError_t launch_sweep_cl(const Consts& c, const StepArgs& a, unsigned grid,
 // sets the kernels' dynamic shared memory limit (once, before any capture)
 cudaError_t prepare_sweep_cl();
 template<int D>
-cudaError_t launch_bi_walls_impl(const Consts& c, const StepArgs& a, cudaStream_t s);
+cudaError_t launch_bi_walls_impl(const Consts& c, const StepArgs& a, unsigned sms,
+                                 cudaStream_t s);
+template<int D>
+cudaError_t launch_sweep_quad_impl(const Consts& c, const StepArgs& a,
+                                   unsigned sms, cudaStream_t s);
 template<int D>
 cudaError_t launch_gather_impl(const Consts& c, const StepArgs& a, cudaStream_t s);
 template<int D>

@@ -62,6 +62,137 @@ k_chunks(const uint32_t* skeys, const uint2* cells, uint32_t N, uint2* chunks,
         chunks[s_count[warp] + __popc(b & ((1u << lane) - 1u))] = w;
 }
 
+// Place of the 64 sub-cells of a cell (4 x 4 x 4, x fastest; 8 x 8 in 2-D)
+// along a Hilbert curve: consecutive places are neighbouring sub-cells
+__constant__ uint8_t kHilbert3[64] = {
+    0, 3, 60, 63, 1, 2, 61, 62, 30, 31, 32, 33, 29, 28, 35, 34,
+    7, 4, 59, 56, 6, 5, 58, 57, 25, 24, 39, 38, 26, 27, 36, 37,
+    8, 11, 52, 55, 15, 12, 51, 48, 16, 23, 40, 47, 19, 20, 43, 44,
+    9, 10, 53, 54, 14, 13, 50, 49, 17, 22, 41, 46, 18, 21, 42, 45
+};
+__constant__ uint8_t kHilbert2[64] = {
+    0, 3, 4, 5, 58, 59, 60, 63, 1, 2, 7, 6, 57, 56, 61, 62,
+    14, 13, 8, 9, 54, 55, 50, 49, 15, 12, 11, 10, 53, 52, 51, 48,
+    16, 17, 30, 31, 32, 33, 46, 47, 19, 18, 29, 28, 35, 34, 45, 44,
+    20, 23, 24, 27, 36, 39, 40, 43, 21, 22, 25, 26, 37, 38, 41, 42
+};
+
+// Clusters of every cell: its particles, ordered along a Hilbert curve
+// through its sub-cells (ties in sorted order), cut every 8 into
+// cperm[first .. end) and clu.  Full clusters wherever the particles lie:
+// groups by octant, which fill clusters of 8 on a lattice, hold 5 to 10
+// particles in a flow that has left it.  A block takes 256 sorted positions,
+// reserves the clusters of the cells that start there with one atomicAdd
+// (the order of the list does not matter) and its warps take those cells.
+constexpr int kClusterThreads = 256;
+template<int D>
+__global__ void __launch_bounds__(kClusterThreads)
+k_cell_clusters(Consts c, StepArgs a, const float4* pos)
+{
+    constexpr int NWARP = kClusterThreads / 32;
+    __shared__ uint4 s_cell[kClusterThreads];  // (first, count, clusters before, -)
+    __shared__ uint32_t s_cnt[NWARP][64];
+    __shared__ uint2 s_warp[NWARP];
+    __shared__ uint32_t s_base;
+    if (__syncthreads_or(threadIdx.x == 0 && a.sc->err))
+        return;  // one read for the whole block
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const uint32_t s0 = blockIdx.x * kClusterThreads + threadIdx.x;
+    uint32_t n = 0;
+    if (s0 < a.N) {
+        const uint32_t key = a.skeys[s0];
+        if (s0 == 0 || a.skeys[s0 - 1] != key)
+            n = a.b.cells[key].y - s0;
+    }
+    const uint32_t ncl = (n + 7u) / 8u;
+    // exclusive scan over the block: cells and clusters
+    uint32_t xc = ncl;
+    const unsigned starts = __ballot_sync(0xffffffffu, n > 0);
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, xc, o);
+        if (lane >= o)
+            xc += y;
+    }
+    if (lane == 31)
+        s_warp[warp] = make_uint2((uint32_t)__popc(starts), xc);
+    __syncthreads();
+    uint32_t cells = 0, clusters = 0, n_cells = 0, n_clusters = 0;
+    for (int w = 0; w < NWARP; w++) {
+        const uint2 v = s_warp[w];
+        if (w < warp) {
+            cells += v.x;
+            clusters += v.y;
+        }
+        n_cells += v.x;
+        n_clusters += v.y;
+    }
+    if (n > 0)
+        s_cell[cells + __popc(starts & lt)] = make_uint4(s0, n, clusters + xc - ncl, 0u);
+    if (threadIdx.x == 0)
+        s_base = n_clusters ? atomicAdd(&a.sc->n_chunks, n_clusters) : 0u;
+    __syncthreads();
+    const uint32_t base = s_base;
+    for (uint32_t w = warp; w < n_cells; w += NWARP) {
+        const uint4 cell = s_cell[w];
+        const uint32_t first = cell.x, cnt = cell.y;
+        for (uint32_t k = lane; k < (cnt + 7u) / 8u; k += 32)
+            a.b.clu[base + cell.z + k] = make_uint2(first + 8u * k, min(8u, cnt - 8u * k));
+        if (cnt <= 8u) {
+            if ((uint32_t)lane < cnt)
+                a.b.cperm[first + lane] = first + lane;
+            continue;
+        }
+        const CaseScalars& cs = a.cs[a.dst.cid[first]];
+        const float scale = (D == 3 ? 4.f : 8.f) * c.idist;
+        auto place = [&](uint32_t s) -> uint32_t {
+            const float4 p = pos[s];
+            const uint32_t x = (uint32_t)((p.x - cs.r_min[0]) * scale);
+            const uint32_t y = (uint32_t)((p.y - cs.r_min[1]) * scale);
+            if (D == 2)
+                return kHilbert2[(x & 7u) | ((y & 7u) << 3)];
+            const uint32_t z = (uint32_t)((p.z - cs.r_min[2]) * scale);
+            return kHilbert3[(x & 3u) | ((y & 3u) << 2) | ((z & 3u) << 4)];
+        };
+        __syncwarp();
+        s_cnt[warp][lane] = 0;
+        s_cnt[warp][32 + lane] = 0;
+        __syncwarp();
+        for (uint32_t b = 0; b < cnt; b += 32) {
+            const bool v = b + lane < cnt;
+            const uint32_t g = v ? place(first + b + lane) : 64u;
+            const unsigned m = __match_any_sync(0xffffffffu, g);
+            if (v && lane == __ffs(m) - 1)
+                s_cnt[warp][g] += (uint32_t)__popc(m);
+            __syncwarp();
+        }
+        // counts -> first positions (lane holds places 2 lane, 2 lane + 1)
+        const uint32_t c0 = s_cnt[warp][2 * lane], c1 = s_cnt[warp][2 * lane + 1];
+        uint32_t x = c0 + c1;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o)
+                x += y;
+        }
+        __syncwarp();
+        s_cnt[warp][2 * lane] = x - c0 - c1;
+        s_cnt[warp][2 * lane + 1] = x - c1;
+        __syncwarp();
+        for (uint32_t b = 0; b < cnt; b += 32) {
+            const bool v = b + lane < cnt;
+            const uint32_t s = first + b + lane;
+            const uint32_t g = v ? place(s) : 64u;
+            const unsigned m = __match_any_sync(0xffffffffu, g);
+            if (v)
+                a.b.cperm[first + s_cnt[warp][g] + (uint32_t)__popc(m & lt)] = s;
+            __syncwarp();
+            if (v && lane == __ffs(m) - 1)
+                s_cnt[warp][g] += (uint32_t)__popc(m);
+            __syncwarp();
+        }
+    }
+}
+
 // End of step of every case: dt = min(dt_var) (Reduction tool), assert
 // dt > 0, t += dt, iter += 1 (set_scalar tools); for a rolling case, the new
 // roll angle and rate at the new time (the reference's motion tools run
@@ -231,10 +362,32 @@ launch_sweep(bool fast, const Consts& c, const StepArgs& a, unsigned grid,
 
 template<int D>
 cudaError_t
-launch_bi_walls(bool fast, const Consts& c, const StepArgs& a, cudaStream_t s)
+launch_clusters(const Consts& c, const StepArgs& a, cudaStream_t s)
 {
-    return fast ? fast::launch_bi_walls_impl<D>(c, a, s)
-                : exact::launch_bi_walls_impl<D>(c, a, s);
+    if (a.N == 0)
+        return cudaSuccess;
+    k_cell_clusters<D><<<(a.N + kClusterThreads - 1) / kClusterThreads,
+                         kClusterThreads, 0, s>>>(
+        c, a, a.clustered ? a.b.rec0 : a.b.posq);
+    return cudaGetLastError();
+}
+
+template<int D>
+cudaError_t
+launch_sweep_quad(bool fast, const Consts& c, const StepArgs& a, unsigned sms,
+                  cudaStream_t s)
+{
+    return fast ? fast::launch_sweep_quad_impl<D>(c, a, sms, s)
+                : exact::launch_sweep_quad_impl<D>(c, a, sms, s);
+}
+
+template<int D>
+cudaError_t
+launch_bi_walls(bool fast, const Consts& c, const StepArgs& a, unsigned sms,
+                cudaStream_t s)
+{
+    return fast ? fast::launch_bi_walls_impl<D>(c, a, sms, s)
+                : exact::launch_bi_walls_impl<D>(c, a, sms, s);
 }
 
 cudaError_t
@@ -275,9 +428,15 @@ launch_export_ihoc(const uint2* cells, uint32_t* ihoc, uint32_t ncap,
 }
 
 template cudaError_t launch_bi_walls<2>(bool, const Consts&, const StepArgs&,
-                                        cudaStream_t);
+                                        unsigned, cudaStream_t);
 template cudaError_t launch_bi_walls<3>(bool, const Consts&, const StepArgs&,
-                                        cudaStream_t);
+                                        unsigned, cudaStream_t);
+template cudaError_t launch_clusters<2>(const Consts&, const StepArgs&, cudaStream_t);
+template cudaError_t launch_clusters<3>(const Consts&, const StepArgs&, cudaStream_t);
+template cudaError_t launch_sweep_quad<2>(bool, const Consts&, const StepArgs&,
+                                          unsigned, cudaStream_t);
+template cudaError_t launch_sweep_quad<3>(bool, const Consts&, const StepArgs&,
+                                          unsigned, cudaStream_t);
 template cudaError_t launch_motion<2>(const StepArgs&, cudaStream_t);
 template cudaError_t launch_motion<3>(const StepArgs&, cudaStream_t);
 template cudaError_t launch_gather<2>(bool, const Consts&, const StepArgs&, cudaStream_t);

@@ -1227,150 +1227,31 @@ k_sweep(Consts c, StepArgs a)
     flush();
 }
 
-// BI walls before the sweep (cfd/BI.xml): for every boundary element, its
-// analytic Shepard factor (BI/Shepard.cl compute: the other elements of the
-// support), the free-slip Laplacian of the fluid velocity (BI/LapU.cl), the
-// pressure gradient it implies (BI/GradP.cl), the pressure interpolated
-// from the fluid (BI/Interpolation.cl, a second pass: it needs that
-// gradient) and its Shepard renormalisation with the density from the
-// linear EOS (BI/InterpolationShepard.cl).  The sweep then reads the
-// elements' pressure from the packed records.
+#include "sweep_quad.cuh"
+
 template<int D>
-__global__ void __launch_bounds__(128)
-k_bi_walls(Consts c, StepArgs a)
+cudaError_t
+launch_bi_walls_impl(const Consts& c, const StepArgs& a, unsigned sms,
+                     cudaStream_t s)
 {
-    constexpr int VS = Vec<D>::VS;
-    constexpr int NC = (D == 3) ? 27 : 9;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.N || a.sc->err)
-        return;
-    const float4 pi = a.b.posq[i];
-    if (__float_as_int(pi.w) != -3)
-        return;
-    const VarSet& T = a.dst;
-    const CaseScalars& cas = a.cs[T.cid[i]];
-    const uint32_t nx = cas.n_cells[0];
-    const uint32_t nxy = cas.n_cells[0] * cas.n_cells[1];
-    const uint32_t key_i = a.skeys[i];
-    const float ri[3] = { pi.x, pi.y, pi.z };
-    const float4 vi = a.b.velq[i];
-    const float ui[3] = { vi.x, vi.y, vi.z };
-    float shep = 1.f;
-    bool self_added = false;
-    float lap[4] = { 0.f, 0.f, 0.f, 0.f };
-    for (int k = 0; k < NC; k++) {
-        const uint2 se = a.b.cells[neighbour_cell<D>(key_i, k, nx, nxy)];
-        for (uint32_t j = se.x; j < se.y; j++) {
-            const float4 pj = a.b.posq[j];
-            const int jm = __float_as_int(pj.w);
-            if (jm == -3) {
-                if (j == i) {
-                    if (!self_added) {
-                        self_added = true;
-                        shep = shep - 0.5f;
-                    }
-                    continue;
-                }
-            } else if (jm != 1) {
-                continue;
-            }
-            float d[3];
-            d[0] = pj.x - ri[0];
-            d[1] = pj.y - ri[1];
-            d[2] = (D == 3) ? pj.z - ri[2] : 0.f;
-            const float q = sqrtf(dot_d<D>(d, d)) / c.H;
-            if (q >= c.SUPPORT)
-                continue;
-            if (jm == 1) {
-                const float4 vj = a.b.velq[j];
-                const float f = kernel_f<D>(q) * c.CONF * a.b.pmq[j].y;
-                const float s2 = f * 2.f / vj.w;
-                lap[0] = lap[0] + s2 * (vj.x - ui[0]);
-                lap[1] = lap[1] + s2 * (vj.y - ui[1]);
-                if (D == 3)
-                    lap[2] = lap[2] + s2 * (vj.z - ui[2]);
-                continue;
-            }
-            float nj[3], tj[3], bj[3];
-            load_normal<D>(T.normal, j, nj);
-            load_normal<D>(T.tangent, j, tj);
-            load_normal<D>(T.binormal, j, bj);
-            const float area = a.b.pmq[j].y;
-            const float rn = dot_d<D>(d, nj);
-            if ((rn > -1e-8f * c.H) && (rn < 1e-8f * c.H)) {
-                if (!self_added) {
-                    const float rt = fabsf(dot_d<D>(d, tj));
-                    const float rb = fabsf(dot_d<D>(d, bj));
-                    const float dr = 0.55f * powf(area, 1.f / (c.DIMS - 1.f));
-                    if ((rt <= dr) && (rb <= dr)) {
-                        self_added = true;
-                        shep = shep - 0.5f;
-                    }
-                }
-                continue;
-            }
-            const float rt = fabsf(dot_d<D>(d, tj));
-            const float rb = fabsf(dot_d<D>(d, bj));
-            shep = shep + (rn * c.CONW * kernel_sp<D>(q) * area +
-                           kernel_sd<D>(fabsf(rn), rt, rb, area));
-        }
-    }
-    // BI/GradP.cl freeslip
-    const uint32_t set_raw = T.iset[i];
-    const uint32_t set = set_raw < c.n_sets ? set_raw : 0u;
-    const float sh = shep < 1.0e-6f ? 1.f : shep;
-    // the dudt Variable: the sorted old rates (midpoint init copy) or, under
-    // improved Euler, the unpermuted array (see k_gather)
-    float dudt[4];
-    Vec<D>::load(T.dudt, i, dudt);
-    float gw[4];
-    for (int k = 0; k < VS; k++)
-        gw[k] = c.visc_dyn[set] / c.refd[set] * lap[k] / sh + c.g[k] - dudt[k];
-    // BI/Interpolation.cl
-    const float rho_i = vi.w;
-    float gpi[3];
-    for (int k = 0; k < 3; k++)
-        gpi[k] = rho_i * gw[k];
-    float p = 0.f;
-    for (int k = 0; k < NC; k++) {
-        const uint2 se = a.b.cells[neighbour_cell<D>(key_i, k, nx, nxy)];
-        for (uint32_t j = se.x; j < se.y; j++) {
-            const float4 pj = a.b.posq[j];
-            if (__float_as_int(pj.w) != 1)
-                continue;
-            float d[3];
-            d[0] = pj.x - ri[0];
-            d[1] = pj.y - ri[1];
-            d[2] = (D == 3) ? pj.z - ri[2] : 0.f;
-            const float q = sqrtf(dot_d<D>(d, d)) / c.H;
-            if (q >= c.SUPPORT)
-                continue;
-            const float2 pm = a.b.pmq[j];
-            const float w = kernel_w<D>(q) * c.CONW * pm.y / a.b.velq[j].w;
-            p = p + (pm.x - dot_d<D>(gpi, d)) * w;
-        }
-    }
-    // BI/InterpolationShepard.cl
-    p = p / sh;
-    const float rho = c.refd[set] + (p - c.p0) / (c.cs * c.cs);
-    T.p[i] = p;
-    T.rho[i] = rho;
-    a.b.pmq[i].x = p;
-    if (a.b.shepard)
-        a.b.shepard[i] = shep;
-    if (a.extras) {
-        Vec<D>::store(a.b.lap_u, i, lap);
-        Vec<D>::store(a.b.grad_p, i, gw);
-    }
+    if (a.N == 0)
+        return cudaSuccess;
+    k_bi_walls<D><<<sms * (16u / kQuadWarps), kQuadWarps * 32, 0, s>>>(c, a);
+    return cudaGetLastError();
 }
 
 template<int D>
 cudaError_t
-launch_bi_walls_impl(const Consts& c, const StepArgs& a, cudaStream_t s)
+launch_sweep_quad_impl(const Consts& c, const StepArgs& a, unsigned sms,
+                       cudaStream_t s)
 {
     if (a.N == 0)
         return cudaSuccess;
-    k_bi_walls<D><<<(a.N + 127) / 128, 128, 0, s>>>(c, a);
+    const unsigned grid = sms * (24u / kQuadWarps);
+    if (c.boundary == AQUA_BOUNDARY_BI)
+        k_sweep_quad<D, true><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
+    else
+        k_sweep_quad<D, false><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
     return cudaGetLastError();
 }
 
@@ -1394,12 +1275,6 @@ launch_sweep_impl(const Consts& c, const StepArgs& a, unsigned grid,
 {
     if (a.N == 0)
         return cudaSuccess;
-    if (c.boundary == AQUA_BOUNDARY_BI) {
-        // one launch shape for the BI walls: the direct sweep with prefetch
-        // and the register budget of 28 resident warps per SM
-        k_sweep<D, 64, 1, uint32_t, true, true, kSweepDirect, 28><<<grid, 64, 0, s>>>(c, a);
-        return cudaGetLastError();
-    }
     switch (variant) {
     case 1:
         k_sweep<D, 64, 128, uint16_t, false, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
@@ -1452,8 +1327,10 @@ launch_sweep_impl(const Consts& c, const StepArgs& a, unsigned grid,
     return cudaGetLastError();
 }
 
-template cudaError_t launch_bi_walls_impl<2>(const Consts&, const StepArgs&, cudaStream_t);
-template cudaError_t launch_bi_walls_impl<3>(const Consts&, const StepArgs&, cudaStream_t);
+template cudaError_t launch_bi_walls_impl<2>(const Consts&, const StepArgs&, unsigned, cudaStream_t);
+template cudaError_t launch_bi_walls_impl<3>(const Consts&, const StepArgs&, unsigned, cudaStream_t);
+template cudaError_t launch_sweep_quad_impl<2>(const Consts&, const StepArgs&, unsigned, cudaStream_t);
+template cudaError_t launch_sweep_quad_impl<3>(const Consts&, const StepArgs&, unsigned, cudaStream_t);
 template cudaError_t launch_gather_impl<2>(const Consts&, const StepArgs&, cudaStream_t);
 template cudaError_t launch_gather_impl<3>(const Consts&, const StepArgs&, cudaStream_t);
 template cudaError_t launch_sweep_impl<2>(const Consts&, const StepArgs&, unsigned,

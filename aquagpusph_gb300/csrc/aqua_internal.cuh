@@ -55,6 +55,7 @@ struct Consts
     float w_conw;       // W factor of the Wendland kernel * CONW
     float f_conf;       // F factor * CONF
     float f_over_w;     // f_conf / w_conw (clustered sweep)
+    uint32_t quad_ok;   // H, CONW and CONF are in the range of quad_div
     // test-only: a bounded wait that completed is reported as timed out
     // (AQUA_ERR_TIMEOUT), so the error path runs with nothing in flight
     uint32_t debug_fake_timeout;

@@ -138,6 +138,7 @@ struct StepArgs
     int extras;        // write the intermediate operators
     int clustered;     // the gather writes rec0/rec1 and the cell list for
                        // the clustered sweep instead of posq/velq/pmq
+    uint32_t cluster;  // particles per cluster of the quad sweep (4 or 8)
 };
 // gather / sweep of the step in the exact (IEEE, no FMA) or fast
 // (-use_fast_math) compilation

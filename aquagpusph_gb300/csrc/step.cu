@@ -78,7 +78,7 @@ __constant__ uint8_t kHilbert2[64] = {
 };
 
 // Clusters of every cell: its particles, ordered along a Hilbert curve
-// through its sub-cells (ties in sorted order), cut every 8 into
+// through its sub-cells (ties in sorted order), cut every 8 (or 4) into
 // cperm[first .. end) and clu.  Full clusters wherever the particles lie:
 // groups by octant, which fill clusters of 8 on a lattice, hold 5 to 10
 // particles in a flow that has left it.  A block takes 256 sorted positions,
@@ -105,7 +105,8 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
         if (s0 == 0 || a.skeys[s0 - 1] != key)
             n = a.b.cells[key].y - s0;
     }
-    const uint32_t ncl = (n + 7u) / 8u;
+    const uint32_t P = a.cluster;  // 4 or 8
+    const uint32_t ncl = (n + P - 1u) / P;
     // exclusive scan over the block: cells and clusters
     uint32_t xc = ncl;
     const unsigned starts = __ballot_sync(0xffffffffu, n > 0);
@@ -136,9 +137,9 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
     for (uint32_t w = warp; w < n_cells; w += NWARP) {
         const uint4 cell = s_cell[w];
         const uint32_t first = cell.x, cnt = cell.y;
-        for (uint32_t k = lane; k < (cnt + 7u) / 8u; k += 32)
-            a.b.clu[base + cell.z + k] = make_uint2(first + 8u * k, min(8u, cnt - 8u * k));
-        if (cnt <= 8u) {
+        for (uint32_t k = lane; k < (cnt + P - 1u) / P; k += 32)
+            a.b.clu[base + cell.z + k] = make_uint2(first + P * k, min(P, cnt - P * k));
+        if (cnt <= P) {
             if ((uint32_t)lane < cnt)
                 a.b.cperm[first + lane] = first + lane;
             continue;

@@ -77,6 +77,13 @@ cp_async_8(void* smem, const void* gmem)
                  :: "r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void
+cp_async_4(void* smem, const void* gmem)
+{
+    const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n"
+                 :: "r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void
 cp_async_commit()
 {
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -1236,7 +1243,11 @@ launch_bi_walls_impl(const Consts& c, const StepArgs& a, unsigned sms,
 {
     if (a.N == 0)
         return cudaSuccess;
-    k_bi_walls<D><<<sms * (16u / kQuadWarps), kQuadWarps * 32, 0, s>>>(c, a);
+    const unsigned grid = sms * (16u / kQuadWarps);
+    if (a.cluster == 4)
+        k_bi_walls<D, 4><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
+    else
+        k_bi_walls<D, 8><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
     return cudaGetLastError();
 }
 
@@ -1248,10 +1259,10 @@ launch_sweep_quad_impl(const Consts& c, const StepArgs& a, unsigned sms,
     if (a.N == 0)
         return cudaSuccess;
     const unsigned grid = sms * (24u / kQuadWarps);
-    if (c.boundary == AQUA_BOUNDARY_BI)
-        k_sweep_quad<D, true><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
-    else
-        k_sweep_quad<D, false><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
+    const bool bi = c.boundary == AQUA_BOUNDARY_BI, small = a.cluster == 4;
+    auto kernel = bi ? (small ? k_sweep_quad<D, true, 4> : k_sweep_quad<D, true, 8>)
+                     : (small ? k_sweep_quad<D, false, 4> : k_sweep_quad<D, false, 8>);
+    kernel<<<grid, kQuadWarps * 32, 0, s>>>(c, a);
     return cudaGetLastError();
 }
 

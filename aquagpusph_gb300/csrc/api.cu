@@ -371,7 +371,7 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
     // each with half the pairs (15,602 particles in 3-D: 163 against 197 us a
     // step; 8,206 in 2-D: 67 against 69).  Above, the shared list of 8 wins
     // (46,545 in 2-D: 149 against 156; 406,402 in 3-D: 1.91 against 2.17 ms).
-    a.cluster = N <= (uint32_t)x->sms * 16u * 8u ? 4u : 8u;
+    a.cluster = !clustered && N <= (uint32_t)x->sms * 16u * 8u ? 4u : 8u;
     Consts cst = x->consts;
     cst.debug_fake_timeout = g_debug_fake_timeout ? 1u : 0u;
     if (x->profiling)
@@ -380,11 +380,13 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
         AQ_CUDA(launch_gather<3>(x->fast, x->consts, a, s));
     else
         AQ_CUDA(launch_gather<2>(x->fast, x->consts, a, s));
+    if (x->profiling)
+        AQ_CUDA(cudaEventRecordWithFlags(x->ev[2], s, cudaEventRecordExternal));
     // the quad sweep: BI walls, and wherever a clustered choice (the default)
     // is set but the clustered sweep does not apply
     const bool bi = x->consts.boundary == AQUA_BOUNDARY_BI;
     const bool quad = !clustered && (bi || x->sweep_variant >= kSweepClustered);
-    if (quad) {
+    if (quad || clustered) {
         if (x->dims == 3)
             AQ_CUDA(launch_clusters<3>(x->consts, a, s));
         else
@@ -396,11 +398,8 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
         else
             AQ_CUDA(launch_bi_walls<2>(x->fast, x->consts, a, (unsigned)x->sms, s));
     }
-    if (x->profiling)
-        AQ_CUDA(cudaEventRecordWithFlags(x->ev[2], s, cudaEventRecordExternal));
     if (clustered) {
-        AQ_CUDA(fast::launch_sweep_cl(cst, a, x->sweep_grid, x->sweep_variant,
-                                      (unsigned)x->sms, s));
+        AQ_CUDA(fast::launch_sweep_cl(cst, a, x->sweep_grid, s));
     } else if (quad) {
         if (x->dims == 3)
             AQ_CUDA(launch_sweep_quad<3>(x->fast, cst, a, (unsigned)x->sms, s));

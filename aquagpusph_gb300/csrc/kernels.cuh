@@ -203,9 +203,9 @@ cudaError_t launch_sweep_impl(const Consts& c, const StepArgs& a, unsigned grid,
                               int variant, cudaStream_t s);
 }  // namespace exact
 namespace fast {
-// clustered sweep: the cluster list then the sweep (variant >= kSweepClustered)
+// the clustered sweep over the cells of launch_clusters()
 cudaError_t launch_sweep_cl(const Consts& c, const StepArgs& a, unsigned grid,
-                            int variant, unsigned sms, cudaStream_t s);
+                            cudaStream_t s);
 // sets the kernels' dynamic shared memory limit (once, before any capture)
 cudaError_t prepare_sweep_cl();
 template<int D>

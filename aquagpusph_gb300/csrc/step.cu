@@ -82,16 +82,23 @@ __constant__ uint8_t kHilbert2[64] = {
 // cperm[first .. end) and clu.  Full clusters wherever the particles lie:
 // groups by octant, which fill clusters of 8 on a lattice, hold 5 to 10
 // particles in a flow that has left it.  A block takes 256 sorted positions,
-// reserves the clusters of the cells that start there with one atomicAdd
-// (the order of the list does not matter) and its warps take those cells.
+// reserves list entries for the cells that start there with one atomicAdd
+// (the order of the lists does not matter) and its warps take those cells.
+//
+// CELLS = false (quad sweep): clu is the work list, in any order.
+// CELLS = true (clustered sweep, 3-D): the work list holds cells (work, wcl);
+// a cell's clusters take the slots of clu from its first sorted index on,
+// probes come last, in clusters of their own, and crow holds the cell's
+// neighbourhood as 9 rows of 3 cells.
 constexpr int kClusterThreads = 256;
-template<int D>
+template<int D, bool CELLS>
 __global__ void __launch_bounds__(kClusterThreads)
 k_cell_clusters(Consts c, StepArgs a, const float4* pos)
 {
     constexpr int NWARP = kClusterThreads / 32;
+    constexpr uint32_t kProbes = 64;  // place of the probes (CELLS)
     __shared__ uint4 s_cell[kClusterThreads];  // (first, count, clusters before, -)
-    __shared__ uint32_t s_cnt[NWARP][64];
+    __shared__ uint32_t s_cnt[NWARP][66];
     __shared__ uint2 s_warp[NWARP];
     __shared__ uint32_t s_base;
     if (__syncthreads_or(threadIdx.x == 0 && a.sc->err))
@@ -131,65 +138,114 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
     if (n > 0)
         s_cell[cells + __popc(starts & lt)] = make_uint4(s0, n, clusters + xc - ncl, 0u);
     if (threadIdx.x == 0)
-        s_base = n_clusters ? atomicAdd(&a.sc->n_chunks, n_clusters) : 0u;
+        s_base = n_cells ? atomicAdd(&a.sc->n_chunks, CELLS ? n_cells : n_clusters) : 0u;
     __syncthreads();
     const uint32_t base = s_base;
     for (uint32_t w = warp; w < n_cells; w += NWARP) {
         const uint4 cell = s_cell[w];
         const uint32_t first = cell.x, cnt = cell.y;
-        for (uint32_t k = lane; k < (cnt + P - 1u) / P; k += 32)
-            a.b.clu[base + cell.z + k] = make_uint2(first + P * k, min(P, cnt - P * k));
-        if (cnt <= P) {
-            if ((uint32_t)lane < cnt)
-                a.b.cperm[first + lane] = first + lane;
-            continue;
+        const uint32_t kc = a.dst.cid[first];
+        const CaseScalars& cs = a.cs[kc];
+        // row (dy, dz) = (lane % 3 - 1, lane / 3 - 1) of the neighbourhood:
+        // cells x-1 .. x+1, as one run of sorted indices (lanes 0-8; the cell
+        // table is read here and the row written after the clusters, so the
+        // loads overlap the work below)
+        uint2 rc3[3] = { make_uint2(1u, 0u), make_uint2(1u, 0u), make_uint2(1u, 0u) };
+        uint32_t key = 0;
+        if (CELLS) {
+            key = a.skeys[first];
+            if (lane < 9) {
+                const uint32_t nx = cs.n_cells[0];
+                const uint32_t nxy = cs.n_cells[0] * cs.n_cells[1];
+                const uint32_t k0 = key + (uint32_t)(lane % 3 - 1) * nx +
+                                    (uint32_t)(lane / 3 - 1) * nxy - 1u;
+                for (int d = 0; d < 3; d++)
+                    rc3[d] = a.b.cells[k0 + d];
+            }
         }
-        const CaseScalars& cs = a.cs[a.dst.cid[first]];
-        const float scale = (D == 3 ? 4.f : 8.f) * c.idist;
-        auto place = [&](uint32_t s) -> uint32_t {
-            const float4 p = pos[s];
-            const uint32_t x = (uint32_t)((p.x - cs.r_min[0]) * scale);
-            const uint32_t y = (uint32_t)((p.y - cs.r_min[1]) * scale);
-            if (D == 2)
-                return kHilbert2[(x & 7u) | ((y & 7u) << 3)];
-            const uint32_t z = (uint32_t)((p.z - cs.r_min[2]) * scale);
-            return kHilbert3[(x & 3u) | ((y & 3u) << 2) | ((z & 3u) << 4)];
-        };
-        __syncwarp();
-        s_cnt[warp][lane] = 0;
-        s_cnt[warp][32 + lane] = 0;
-        __syncwarp();
-        for (uint32_t b = 0; b < cnt; b += 32) {
-            const bool v = b + lane < cnt;
-            const uint32_t g = v ? place(first + b + lane) : 64u;
-            const unsigned m = __match_any_sync(0xffffffffu, g);
-            if (v && lane == __ffs(m) - 1)
-                s_cnt[warp][g] += (uint32_t)__popc(m);
+        uint32_t probes = 0;
+        if (cnt > P || CELLS) {
+            const float scale = (D == 3 ? 4.f : 8.f) * c.idist;
+            auto place = [&](uint32_t s) -> uint32_t {
+                if (CELLS && a.dst.imove[s] == 0)
+                    return kProbes;
+                const float4 p = pos[s];
+                const uint32_t x = (uint32_t)((p.x - cs.r_min[0]) * scale);
+                const uint32_t y = (uint32_t)((p.y - cs.r_min[1]) * scale);
+                if (D == 2)
+                    return kHilbert2[(x & 7u) | ((y & 7u) << 3)];
+                const uint32_t z = (uint32_t)((p.z - cs.r_min[2]) * scale);
+                return kHilbert3[(x & 3u) | ((y & 3u) << 2) | ((z & 3u) << 4)];
+            };
             __syncwarp();
+            s_cnt[warp][lane] = 0;
+            s_cnt[warp][32 + lane] = 0;
+            if (lane == 0)
+                s_cnt[warp][kProbes] = 0;
+            __syncwarp();
+            for (uint32_t b = 0; b < cnt; b += 32) {
+                const bool v = b + lane < cnt;
+                const uint32_t g = v ? place(first + b + lane) : kProbes + 1u;
+                const unsigned m = __match_any_sync(0xffffffffu, g);
+                if (v && lane == __ffs(m) - 1)
+                    s_cnt[warp][g] += (uint32_t)__popc(m);
+                __syncwarp();
+            }
+            // counts -> first positions (lane holds places 2 lane, 2 lane + 1)
+            const uint32_t c0 = s_cnt[warp][2 * lane], c1 = s_cnt[warp][2 * lane + 1];
+            probes = s_cnt[warp][kProbes];
+            uint32_t x = c0 + c1;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o)
+                    x += y;
+            }
+            __syncwarp();
+            s_cnt[warp][2 * lane] = x - c0 - c1;
+            s_cnt[warp][2 * lane + 1] = x - c1;
+            if (lane == 0)
+                s_cnt[warp][kProbes] = cnt - probes;
+            __syncwarp();
+            for (uint32_t b = 0; b < cnt; b += 32) {
+                const bool v = b + lane < cnt;
+                const uint32_t s = first + b + lane;
+                const uint32_t g = v ? place(s) : kProbes + 1u;
+                const unsigned m = __match_any_sync(0xffffffffu, g);
+                if (v)
+                    a.b.cperm[first + s_cnt[warp][g] + (uint32_t)__popc(m & lt)] = s;
+                __syncwarp();
+                if (v && lane == __ffs(m) - 1)
+                    s_cnt[warp][g] += (uint32_t)__popc(m);
+                __syncwarp();
+            }
+        } else if ((uint32_t)lane < cnt) {
+            a.b.cperm[first + lane] = first + lane;
         }
-        // counts -> first positions (lane holds places 2 lane, 2 lane + 1)
-        const uint32_t c0 = s_cnt[warp][2 * lane], c1 = s_cnt[warp][2 * lane + 1];
-        uint32_t x = c0 + c1;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o)
-                x += y;
+        // clusters of the others, then of the probes; at most as many as
+        // particles
+        const uint32_t n0 = cnt - probes, k0 = (n0 + P - 1u) / P;
+        const uint32_t nk = k0 + (probes + P - 1u) / P;
+        const uint32_t slot0 = CELLS ? first : base + cell.z;
+        for (uint32_t k = lane; k < nk; k += 32) {
+            const uint32_t at = k < k0 ? P * k : n0 + P * (k - k0);
+            a.b.clu[slot0 + k] = make_uint2(first + at, min(P, (k < k0 ? n0 : cnt) - at));
         }
-        __syncwarp();
-        s_cnt[warp][2 * lane] = x - c0 - c1;
-        s_cnt[warp][2 * lane + 1] = x - c1;
-        __syncwarp();
-        for (uint32_t b = 0; b < cnt; b += 32) {
-            const bool v = b + lane < cnt;
-            const uint32_t s = first + b + lane;
-            const uint32_t g = v ? place(s) : 64u;
-            const unsigned m = __match_any_sync(0xffffffffu, g);
-            if (v)
-                a.b.cperm[first + s_cnt[warp][g] + (uint32_t)__popc(m & lt)] = s;
-            __syncwarp();
-            if (v && lane == __ffs(m) - 1)
-                s_cnt[warp][g] += (uint32_t)__popc(m);
-            __syncwarp();
+        if (CELLS) {
+            if (lane == 0) {
+                a.b.work[base + w] = make_uint2(key, first);
+                a.b.wcl[base + w] = make_uint4(first, first + cnt, kc, nk);
+            }
+            if (lane < 9) {
+                uint32_t lo = 0xffffffffu, hi = 0;
+                for (int d = 0; d < 3; d++) {
+                    if (rc3[d].x < rc3[d].y) {
+                        lo = min(lo, rc3[d].x);
+                        hi = max(hi, rc3[d].y);
+                    }
+                }
+                a.b.crow[(size_t)(base + w) * 9 + lane] =
+                    hi > lo ? make_uint2(lo, hi - lo) : make_uint2(0u, 0u);
+            }
         }
     }
 }
@@ -367,9 +423,11 @@ launch_clusters(const Consts& c, const StepArgs& a, cudaStream_t s)
 {
     if (a.N == 0)
         return cudaSuccess;
-    k_cell_clusters<D><<<(a.N + kClusterThreads - 1) / kClusterThreads,
-                         kClusterThreads, 0, s>>>(
-        c, a, a.clustered ? a.b.rec0 : a.b.posq);
+    const unsigned grid = (a.N + kClusterThreads - 1) / kClusterThreads;
+    if (D == 3 && a.clustered)
+        k_cell_clusters<3, true><<<grid, kClusterThreads, 0, s>>>(c, a, a.b.rec0);
+    else
+        k_cell_clusters<D, false><<<grid, kClusterThreads, 0, s>>>(c, a, a.b.posq);
     return cudaGetLastError();
 }
 

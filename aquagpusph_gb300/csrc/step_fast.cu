@@ -13,60 +13,27 @@ namespace fast {
 #include "sweep_cl.cuh"
 #undef AQUA_FAST_ARITH
 
-namespace {
-
-template<int NW, int CAP, int MINB>
-cudaError_t
-launch_cl(const Consts& c, const StepArgs& a, unsigned grid, unsigned sms,
-          cudaStream_t s)
-{
-    constexpr uint32_t kPer = kCellListThreads * kCellListItems;
-    k_cell_list<<<max(1u, (a.N + kPer - 1) / kPer), kCellListThreads, 0, s>>>(
-        a.skeys, a.N, a.b.cells, a.dst.cid, a.b.work, a.b.wcl, a.sc);
-    k_clusters<<<sms * 8u, 256, 0, s>>>(c, a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess)
-        return e;
-    k_sweep_cl<NW, CAP, MINB><<<grid, NW * 32, sizeof(ClSmem<NW, CAP>), s>>>(c, a);
-    return cudaGetLastError();
-}
-
-template<int NW, int CAP, int MINB>
-cudaError_t
-prepare_cl()
-{
-    return cudaFuncSetAttribute(k_sweep_cl<NW, CAP, MINB>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(ClSmem<NW, CAP>));
-}
-
-}  // namespace
+// blocks of 8 warps, 3 per SM (shared memory, registers), 2,048 staged
+// records per pass
+constexpr int kClWarps = 8, kClRecords = 2048;
 
 cudaError_t
-launch_sweep_cl(const Consts& c, const StepArgs& a, unsigned grid, int variant,
-                unsigned sms, cudaStream_t s)
+launch_sweep_cl(const Consts& c, const StepArgs& a, unsigned grid,
+                cudaStream_t s)
 {
     if (a.N == 0)
         return cudaSuccess;
-    switch (variant) {
-    case kSweepClustered + 0:
-        return launch_cl<8, 2048, 2>(c, a, grid, sms, s);
-    case kSweepClustered + 2:
-        return launch_cl<12, 2048, 2>(c, a, grid, sms, s);
-    default:
-        return launch_cl<8, 2048, 3>(c, a, grid, sms, s);
-    }
+    k_sweep_cl<kClWarps, kClRecords, 3>
+        <<<grid, kClWarps * 32, sizeof(ClSmem<kClWarps, kClRecords>), s>>>(c, a);
+    return cudaGetLastError();
 }
 
 cudaError_t
 prepare_sweep_cl()
 {
-    cudaError_t e = prepare_cl<8, 2048, 2>();
-    if (e == cudaSuccess)
-        e = prepare_cl<8, 2048, 3>();
-    if (e == cudaSuccess)
-        e = prepare_cl<12, 2048, 2>();
-    return e;
+    return cudaFuncSetAttribute(k_sweep_cl<kClWarps, kClRecords, 3>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(ClSmem<kClWarps, kClRecords>));
 }
 
 }  // namespace fast

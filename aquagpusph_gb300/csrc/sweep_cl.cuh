@@ -12,30 +12,26 @@
 // nine contiguous runs of sorted particles (one per (dy, dz) row: the cell
 // keys run x-fastest).
 //
-// Clusters: k_clusters groups each cell's particles by octant into
-// clusters of at most 8 (small octant groups merge).  A warp takes one
-// cluster at a time as 8 particles x 4 neighbour slots: lane l holds
-// particle l % 8 and takes every fourth neighbour of the cluster's list from
-// slot l / 8 on, so that the 8 lanes of one phase of a 16-byte shared load
-// read the same record (a broadcast, free of bank conflicts).
-// The list holds the staged candidates within the support of the octant
-// boxes of the cluster's particles.  After each staging the block
-// classifies every staged record once into a 16-bit mask: the octant boxes
-// of the cell it comes within the support of (a box per octant, spanning,
-// per axis and half, the cell's particles there), in the low byte for a
-// fluid record and the high byte for a boundary element.  Each cluster then
-// scans those masks and compacts its candidates with ballots.  About 60% of the evaluated pairs lie in the support on a
-// lattice, against about a third of the lanes in k_sweep.  Pairs outside
-// the support add exact zeros (the kernel factor is cut to zero at
-// q >= SUPPORT), so the lists only have to be conservative: each octant
-// box holds its particles.  The four partial sums of a particle are added
-// by two butterfly shuffles.
+// Clusters: k_cell_clusters orders each cell's particles along a Hilbert
+// curve and cuts them every 8.  A warp takes one cluster at a time as 8
+// particles x 4 neighbour slots: lane l holds particle l % 8 and takes every
+// fourth neighbour of the cluster's list from slot l / 8 on, so that the 8
+// lanes of one phase of a 16-byte shared load read the same record (a
+// broadcast, free of bank conflicts).  The list holds the staged records
+// within the support of the box of the cluster's particles, tested by the
+// warp, two per lane, and compacted with ballots.  Pairs outside the support
+// add exact zeros (the kernel factor is cut to zero at the support), so the
+// box only has to be conservative.  The summation order is not the
+// reference's (staging order, four interleaved partial sums): this sweep is
+// the fast build's, checked within the per-step rate tolerance 1e-5.  It is
+// deterministic: clusters, lists, parts and staging depend on the sorted
+// state only, not on the launch shape.
 //
-// Summation order differs from the reference's (neighbours in staging
-// order, four interleaved partial sums): this sweep is the fast build's,
-// checked within the per-step rate tolerance 1e-5.  It is deterministic:
-// clusters, lists and staging depend on the sorted state only, not on the
-// launch shape.
+// The last n_cl mod 8 clusters of a cell are each shared by 8 / (n_cl mod 8)
+// warps (rounded down), which take equal parts of the staged records; the
+// first warps add the parts in order and finish those clusters.  Off the
+// lattice most cells hold 9 clusters, and seven warps would wait for the
+// ninth.
 //
 // Boundary elements reach fluid particles through a second list (the BIe
 // wall sums), which also serves the elastic bounce and PST of the
@@ -54,14 +50,13 @@
 
 namespace {
 
-constexpr int kClListCap = 192;      // fluid survivors per warp (128 per round
-                                     // of the mask scan, drained above 64)
+constexpr int kClListCap = 192;      // fluid survivors per warp (64 per round
+                                     // of the scan, drained above 128)
 constexpr int kClWallCap = 192;      // boundary-element survivors per warp
-// per staged record: bit o (o < 8) of a fluid record, bit 8 + o of a
-// boundary element = within the support of the cell's octant box o
-constexpr uint32_t kMaskWallShift = 8;
 constexpr int kClMaxPieces = 32;     // staged runs per pass
 constexpr uint32_t kClWaitLimit = 1u << 22;
+constexpr uint32_t kClShare = 8;     // warps that share a cell's last clusters
+constexpr int kClSums = 13;          // sums of a particle
 
 // Shared memory of one block: staged records (CAP + 1: the last is a zero
 // record that pads the lists to whole quads), per-warp lists, staged runs
@@ -72,9 +67,8 @@ struct ClSmem
     float4 r1[CAP + 1];
     uint16_t list[NW][kClListCap + 4];   // + room for the padding quad
     uint16_t wall[NW][kClWallCap + 4];
-    // the staged boundary elements, by warp-sized chunks of the staging
-    alignas(8) uint16_t mask[CAP + 4];  // per staged record: octants by kind
-    float ivl[12];               // octant boxes: axis a, half h: [lo, hi] at 4 a + 2 h
+    float part[kClShare][kClSums][8];    // sums of a shared cluster, by part
+    uint32_t wn[NW];                     // entries of wall[]; bit 31: overflowed
     uint4 piece[kClMaxPieces];   // (slot, sorted first, count, -)
     uint2 row[9];                // (sorted first, count) of each row
     uint32_t npieces;
@@ -84,225 +78,24 @@ struct ClSmem
     uint64_t mbar;
 };
 
-// Octant (0-7, x fastest) of a position inside its cell: the halves of the
-// cell along each axis (cells are (support h) wide from the case's r_min)
-__device__ __forceinline__ uint32_t
-cl_octant(const float4 p, const CaseScalars& cs, float sc2)
-{
-    const uint32_t ox = (uint32_t)((p.x - cs.r_min[0]) * sc2) & 1u;
-    const uint32_t oy = (uint32_t)((p.y - cs.r_min[1]) * sc2) & 1u;
-    const uint32_t oz = (uint32_t)((p.z - cs.r_min[2]) * sc2) & 1u;
-    return ox | (oy << 1) | (oz << 2);
-}
-
-// The cells holding particles, as (key, first sorted index), and their
-// (first, end, -, case) in the cluster table: position s starts a cell
-// where the sorted key changes.  A block takes
-// kCellListThreads x kCellListItems positions and reserves its entries with
-// one atomicAdd (the order of the list does not matter: every cell is swept
-// the same wherever it sits in it).
-constexpr int kCellListThreads = 1024;
-constexpr int kCellListItems = 8;
-__global__ void __launch_bounds__(kCellListThreads)
-k_cell_list(const uint32_t* skeys, uint32_t N, const uint2* cells,
-            const uint32_t* cid, uint2* work, uint4* wcl, DevScalars* sc)
-{
-    __shared__ uint32_t s_warp[kCellListThreads / 32];
-    __shared__ uint32_t s_base;
-    if (__syncthreads_or(threadIdx.x == 0 && sc->err))
-        return;  // one read for the whole block
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t base = blockIdx.x * (uint32_t)(kCellListThreads * kCellListItems);
-    uint32_t starts = 0;  // bit it: position base + it * threads + t starts a cell
-    for (int it = 0; it < kCellListItems; it++) {
-        const uint32_t s = base + it * kCellListThreads + threadIdx.x;
-        if (s < N && (s == 0 || skeys[s - 1] != skeys[s]))
-            starts |= 1u << it;
-    }
-    // block-wide exclusive scan of the counts
-    const uint32_t v = (uint32_t)__popc(starts);
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o)
-            x += y;
-    }
-    if (lane == 31)
-        s_warp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = s_warp[lane];
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o)
-                w += y;
-        }
-        s_warp[lane] = w;  // inclusive warp totals
-        if (lane == 31)
-            s_base = w ? atomicAdd(&sc->n_chunks, w) : 0u;
-    }
-    __syncthreads();
-    uint32_t o = s_base + (warp > 0 ? s_warp[warp - 1] : 0u) + x - v;
-    for (int it = 0; it < kCellListItems; it++) {
-        if (starts & (1u << it)) {
-            const uint32_t s = base + it * kCellListThreads + threadIdx.x;
-            const uint32_t key = skeys[s];
-            work[o] = make_uint2(key, s);
-            // (first, end, -, case) for k_clusters, which completes it
-            wcl[o] = make_uint4(s, cells[key].y, 0u, cid[s]);
-            o++;
-        }
-    }
-}
-
-// Clusters of every cell in the work list: one warp per cell.  The cell's
-// particles are ordered by group (octants 0-7 of the cell, then probes) into
-// cperm[first .. end) and cut into clusters: a group joins the open cluster
-// when it fits whole, else it starts new ones of 8 (probes always start a
-// new cluster).  Ranks within a group follow the sorted order, so the
-// clusters are a function of the sorted state.
-__global__ void __launch_bounds__(256)
-k_clusters(Consts c, StepArgs a)
-{
-    __shared__ uint32_t s_cnt[8][16];
-    __shared__ uint32_t s_pos[8][16];
-    if (a.sc->err)
-        return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t n_work = a.sc->n_chunks;
-    const uint32_t lt = (1u << lane) - 1u;
-    for (uint32_t w = blockIdx.x * 8u + warp; w < n_work; w += gridDim.x * 8u) {
-        const uint4 wc0 = a.b.wcl[w];  // (first, end, -, case) of k_cell_list
-        const uint32_t first = wc0.x;
-        const uint32_t end = wc0.y;
-        const uint32_t n = end - first;
-        const CaseScalars& cs = a.cs[wc0.w];
-        // row (dy, dz) = (lane % 3 - 1, lane / 3 - 1) of the sweep's
-        // neighbourhood: cells x-1 .. x+1, as one run of sorted indices
-        // (lanes 0-8; the cell table is read here and the row written after
-        // the clusters, so the loads overlap the work below)
-        uint2 rc3[3] = { make_uint2(1u, 0u), make_uint2(1u, 0u), make_uint2(1u, 0u) };
-        if (lane < 9) {
-            const uint32_t key = a.b.work[w].x;
-            const uint32_t nx = cs.n_cells[0];
-            const uint32_t nxy = cs.n_cells[0] * cs.n_cells[1];
-            const uint32_t k0 = key + (uint32_t)(lane % 3 - 1) * nx +
-                                (uint32_t)(lane / 3 - 1) * nxy - 1u;
-            for (int d = 0; d < 3; d++)
-                rc3[d] = a.b.cells[k0 + d];
-        }
-        const float sc2 = 2.f * c.idist;
-        auto group = [&](uint32_t s) -> uint32_t {
-            if (a.dst.imove[s] == 0)
-                return 8u;
-            return cl_octant(a.b.rec0[s], cs, sc2);
-        };
-        if (lane < 16)
-            s_cnt[warp][lane] = 0;
-        __syncwarp();
-        for (uint32_t b = 0; b < n; b += 32) {
-            const bool v = b + lane < n;
-            const uint32_t g = v ? group(first + b + lane) : 16u;
-            const unsigned m = __match_any_sync(0xffffffffu, g);
-            if (v && lane == __ffs(m) - 1)
-                s_cnt[warp][g] += (uint32_t)__popc(m);
-            __syncwarp();
-        }
-        if (lane == 0) {
-            // the walk over the groups: counts the clusters, then writes them
-            auto walk = [&](bool write, uint32_t k) -> uint32_t {
-                uint32_t pos = 0, coff = 0, ccnt = 0;
-                bool open = false;
-                for (uint32_t g = 0; g < 9; g++) {
-                    const uint32_t cg = s_cnt[warp][g];
-                    if (write)
-                        s_pos[warp][g] = pos;
-                    if (cg == 0)
-                        continue;
-                    if (open && (g == 8 || ccnt + cg > 8)) {
-                        if (write)
-                            a.b.clu[k] = make_uint2(first + coff, ccnt);
-                        k++;
-                        open = false;
-                    }
-                    if (open) {
-                        ccnt += cg;
-                    } else {
-                        uint32_t left = cg, p = pos;
-                        while (left > 8) {
-                            if (write)
-                                a.b.clu[k] = make_uint2(first + p, 8u);
-                            k++;
-                            p += 8;
-                            left -= 8;
-                        }
-                        coff = p;
-                        ccnt = left;
-                        open = true;
-                    }
-                    pos += cg;
-                }
-                if (open) {
-                    if (write)
-                        a.b.clu[k] = make_uint2(first + coff, ccnt);
-                    k++;
-                }
-                return k;
-            };
-            // a cell has at most as many clusters as particles: its
-            // clusters take the slots of clu from its first sorted index on
-            const uint32_t n_cl = walk(true, first) - first;
-            a.b.wcl[w] = make_uint4(first, end, wc0.w, n_cl);
-        }
-        __syncwarp();
-        if (lane < 16)
-            s_cnt[warp][lane] = 0;  // running ranks
-        __syncwarp();
-        for (uint32_t b = 0; b < n; b += 32) {
-            const bool v = b + lane < n;
-            const uint32_t s = first + b + lane;
-            const uint32_t g = v ? group(s) : 16u;
-            const unsigned m = __match_any_sync(0xffffffffu, g);
-            if (v)
-                a.b.cperm[first + s_pos[warp][g] + s_cnt[warp][g] +
-                          (uint32_t)__popc(m & lt)] = s;
-            __syncwarp();
-            if (v && lane == __ffs(m) - 1)
-                s_cnt[warp][g] += (uint32_t)__popc(m);
-            __syncwarp();
-        }
-        if (lane < 9) {
-            uint32_t lo = 0xffffffffu, hi = 0;
-            for (int d = 0; d < 3; d++) {
-                if (rc3[d].x < rc3[d].y) {
-                    lo = min(lo, rc3[d].x);
-                    hi = max(hi, rc3[d].y);
-                }
-            }
-            a.b.crow[(size_t)w * 9 + lane] = hi > lo ? make_uint2(lo, hi - lo) : make_uint2(0u, 0u);
-        }
-    }
-}
-
-
 // Everything after the sums for sorted particle i of a cluster (the same
 // steps and expressions as the epilogue of k_sweep): Shepard, the BIe and
 // cfd rates, delta-SPH, elastic bounce, midpoint relax and corrector, PST,
 // the variable time step; returns dt_var (+inf for a lane without a
 // particle).  The four lanes of a particle compute alike; `store` selects
 // the one that writes.  The boundary elements of the elastic bounce and the
-// PST come from the cluster's staged wall list (entries wl[0 .. wfill) of
-// the staged records) or, when `walls_global`, from the per-cell index
-// ranges of the 27 cells around `key` in global memory.
+// PST come from the cluster's staged wall lists (those of warps l0 .. l0 + L
+// - 1, in order) or, when `walls_global`, from the per-cell index ranges of
+// the 27 cells around `key` in global memory.
+template<int NW, int CAP>
 __device__ __forceinline__ float
 sweep_cl_finish(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
                 int im, bool want, bool fluid, bool sensor, bool store,
                 float dt, const float4 r0i, const float4 r1i, float shep,
                 float gp0, float gp1, float gp2, float lu0, float lu1,
                 float lu2, float du, float lp, float gw0, float gw1, float gw2,
-                float dbi, bool walls_global, const uint16_t* wl,
-                uint32_t wfill, const float4* sr0, const float4* sr1,
-                uint32_t key, const CaseScalars& cas)
+                float dbi, bool walls_global, const ClSmem<NW, CAP>& S,
+                uint32_t l0, uint32_t L, uint32_t key, const CaseScalars& cas)
 {
     if (!valid)
         return INFINITY;
@@ -388,11 +181,14 @@ sweep_cl_finish(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
     const uint32_t nxy = cas.n_cells[0] * cas.n_cells[1];
     auto for_walls = [&](auto&& f) {
         if (!walls_global) {
-            for (uint32_t k = 0; k < wfill; k++) {
-                const uint32_t j = wl[k];
-                const float4 pj = sr0[j];
-                const float4 nj = sr1[j];
-                f(pj, nj, -pj.w);
+            for (uint32_t l = l0; l < l0 + L; l++) {
+                const uint32_t n = S.wn[l];
+                for (uint32_t k = 0; k < n; k++) {
+                    const uint32_t j = S.wall[l][k];
+                    const float4 pj = S.r0[j];
+                    const float4 nj = S.r1[j];
+                    f(pj, nj, -pj.w);
+                }
             }
             return;
         }
@@ -611,45 +407,6 @@ k_sweep_cl(Consts c, StepArgs a)
                 atomicOr(&a.sc->err, kErrTimeout);
             return false;
         }
-        // classify the staged records once for all the cell's clusters:
-        // their kind, and which octant boxes of the cell (S.ivl) they come
-        // within the support of (box distance per axis and half, summed
-        // over the 8 combinations)
-        {
-            const uint32_t nst = S.nstaged;
-            float lo[6], hi[6];
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                lo[q] = S.ivl[2 * q];
-                hi[q] = S.ivl[2 * q + 1];
-            }
-            for (uint32_t k = tid; k < nst; k += NW * 32) {
-                const float4 pc = S.r0[k];
-                uint32_t m = 0u;
-                if (pc.w != 0.f) {
-                    const float x[3] = { pc.x, pc.y, pc.z };
-                    float d2[6];
-#pragma unroll
-                    for (int q = 0; q < 6; q++) {
-                        const float d = fmaxf(fmaxf(lo[q] - x[q >> 1], x[q >> 1] - hi[q]), 0.f);
-                        d2[q] = d * d;
-                    }
-                    // (x half, y half) combinations, then z
-                    const float dxy[4] = { d2[0] + d2[2], d2[1] + d2[2],
-                                           d2[0] + d2[3], d2[1] + d2[3] };
-#pragma unroll
-                    for (int o = 0; o < 8; o++)
-                        if (dxy[o & 3] + d2[4 + (o >> 2)] < R2)
-                            m |= 1u << o;
-                    if (pc.w < 0.f)
-                        m <<= kMaskWallShift;
-                }
-                S.mask[k] = (uint16_t)m;
-            }
-            if (tid < 3)
-                S.mask[nst + tid] = 0;  // read with the last records' group of 4
-        }
-        __syncthreads();
         return true;
     };
 
@@ -706,67 +463,32 @@ k_sweep_cl(Consts c, StepArgs a)
         __syncthreads();
         const uint32_t npass = (S.total + CAP - 1) / CAP;
         const bool single = npass <= 1;
-        if (warp == NW - 1) {
-            // the octant boxes of the cell: per axis and half, the extent of
-            // the cell's particles that take neighbour sums (probes apart);
-            // an empty half stays [+inf, -inf] and is never within reach.
-            // Ready before the classification (stage's barrier).
-            const float sc2 = 2.f * c.idist;
-            float bl[6], bh[6];
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                bl[q] = INFINITY;
-                bh[q] = -INFINITY;
-            }
-            for (uint32_t sidx = wc.x + lane; sidx < wc.y; sidx += 32) {
-                const int imv = T.imove[sidx];
-                if (imv < -3 || imv > 1 || imv == 0)
-                    continue;
-                const float4 p = a.b.rec0[sidx];
-                const uint32_t o = cl_octant(p, cas, sc2);
-                const float x[3] = { p.x, p.y, p.z };
-#pragma unroll
-                for (int ax = 0; ax < 3; ax++) {
-                    // constant indices (registers): half 0 or 1 by select
-                    const bool up = (o >> ax) & 1u;
-                    bl[2 * ax] = up ? bl[2 * ax] : fminf(bl[2 * ax], x[ax]);
-                    bh[2 * ax] = up ? bh[2 * ax] : fmaxf(bh[2 * ax], x[ax]);
-                    bl[2 * ax + 1] = up ? fminf(bl[2 * ax + 1], x[ax]) : bl[2 * ax + 1];
-                    bh[2 * ax + 1] = up ? fmaxf(bh[2 * ax + 1], x[ax]) : bh[2 * ax + 1];
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                for (int o = 16; o > 0; o >>= 1) {
-                    bl[q] = fminf(bl[q], __shfl_xor_sync(0xffffffffu, bl[q], o));
-                    bh[q] = fmaxf(bh[q], __shfl_xor_sync(0xffffffffu, bh[q], o));
-                }
-            }
-            if (lane < 6) {
-                float l = bl[0], h = bh[0];
-#pragma unroll
-                for (int q = 1; q < 6; q++)
-                    if (lane == (uint32_t)q) {
-                        l = bl[q];
-                        h = bh[q];
-                    }
-                S.ivl[2 * lane] = l;
-                S.ivl[2 * lane + 1] = h;
-            }
-        }
         bool failed = !stage(0);
         if (tid == 0)
             w_next = fetch();  // consumed at the end of this cell
-        // single pass: each warp takes every NW-th cluster; several passes:
-        // waves of NW clusters, each wave re-staging every pass
-        const uint32_t waves = single ? 1u : (n_cl + NW - 1) / NW;
-        for (uint32_t wave = 0; wave < waves && !failed; wave++) {
-            const uint32_t c_begin = single ? (uint32_t)warp : wave * NW + warp;
-            const uint32_t c_step = single ? (uint32_t)NW : 0xffffffffu;
-            for (uint32_t ci = c_begin; ; ci += c_step) {
-                const bool have = ci < n_cl;
-                if (single && !have)
+        // Single pass: each warp takes every NW-th task, a whole cluster or a
+        // part of one of the last clusters, whose parts are then added and
+        // finished by the first warps.  Several passes: waves of NW whole
+        // clusters, each wave re-staging every pass.
+        const uint32_t rest = n_cl % kClShare;
+        const uint32_t share = single && rest && NW == (int)kClShare ? kClShare / rest : 1u;
+        const uint32_t whole = share > 1u ? n_cl - rest : n_cl;
+        const uint32_t parts = share > 1u ? rest * share : 0u;
+        bool combine = false;
+        for (uint32_t t = warp; !failed; t += NW) {
+            if (single ? t >= whole + parts : t - warp >= n_cl) {
+                if (parts == 0)
                     break;
+                __syncthreads();  // every part is stored
+                if ((uint32_t)warp >= rest)
+                    break;
+                combine = true;
+            }
+            const bool part = parts != 0u && !combine && t >= whole;
+            const uint32_t u = t - whole;  // part
+            const uint32_t ci = combine ? whole + warp : part ? whole + u / share : t;
+            {
+                const bool have = ci < n_cl;
                 // ---- cluster set-up
                 uint2 cl = make_uint2(0u, 0u);
                 if (have)
@@ -782,12 +504,6 @@ k_sweep_cl(Consts c, StepArgs a)
                 const bool any_fluid = __any_sync(0xffffffffu, fluid);
                 const bool probes = __any_sync(0xffffffffu, sensor);
                 const bool any_want = __any_sync(0xffffffffu, want);
-                // the octants of the cluster's particles that take sums: the
-                // candidates are the staged records within the support of
-                // any of those octant boxes (each box holds its particles,
-                // so the list is conservative)
-                const uint32_t omask = __reduce_or_sync(
-                    0xffffffffu, want && !sensor ? 1u << cl_octant(r0i, cas, 2.f * c.idist) : 0u);
                 float shep = 0.f, gp0 = 0.f, gp1 = 0.f, gp2 = 0.f;
                 float lu0 = 0.f, lu1 = 0.f, lu2 = 0.f, du = 0.f, lp = 0.f;
                 float gw0 = 0.f, gw1 = 0.f, gw2 = 0.f, dbi = 0.f;
@@ -857,16 +573,35 @@ k_sweep_cl(Consts c, StepArgs a)
                     }
                 };
 
-                for (uint32_t p = 0; p < npass && !failed; p++) {
-                    if (p > 0 || wave > 0) {  // pass 0 of wave 0 is staged
-                        __syncthreads();
-                        failed = !stage(p);
-                        if (failed)
-                            break;
+                // the box of the cluster's particles that take sums
+                float lo[3], hi[3];
+                {
+                    const float x[3] = { r0i.x, r0i.y, r0i.z };
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        lo[d] = want && !sensor ? x[d] : INFINITY;
+                        hi[d] = want && !sensor ? x[d] : -INFINITY;
+#pragma unroll
+                        for (int o = 4; o > 0; o >>= 1) {
+                            lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                            hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+                        }
+                    }
+                }
+                for (uint32_t p = 0; p < (combine ? 0u : npass) && !failed; p++) {
+                    if (p > 0 || t >= NW) {  // pass 0 of the first wave is staged
+                        if (!single) {
+                            __syncthreads();
+                            failed = !stage(p);
+                            if (failed)
+                                break;
+                        }
                     }
                     if (!have || !any_want)
                         continue;
                     const uint32_t nst = S.nstaged;
+                    if (probes && part && u % share != 0u)
+                        continue;  // the first part sums a probe cluster
                     if (probes) {
                         // probe cluster: lane m < 8 sums probe m over every
                         // staged record (cfd/Sensors.cl: fluid neighbours)
@@ -914,45 +649,36 @@ k_sweep_cl(Consts c, StepArgs a)
                     }
                     uint32_t fill = 0;
                     uint32_t wdone = wfill;  // wall entries already summed
-                    // the boundary elements matter to fluid particles only
-                    const uint32_t wmask = any_fluid ? omask << kMaskWallShift : 0u;
-                    // 128 records per round, four per lane (records 4l ..
-                    // 4l+3), listed in staging order
-                    for (uint32_t base = 0; base < nst; base += 128) {
-                        const uint32_t k0 = base + 4u * lane;
-                        uint2 mm = make_uint2(0u, 0u);
-                        if (k0 < nst)
-                            mm = *reinterpret_cast<const uint2*>(&S.mask[k0]);
-                        const uint32_t m[4] = { mm.x & 0xffffu, mm.x >> 16, mm.y & 0xffffu, mm.y >> 16 };
-                        bool fl[4], wa[4];
-                        unsigned bw[4];
-                        uint32_t before = 0, wbefore = 0, tot = 0, wtot = 0;
+                    const uint32_t g = part ? u % share : 0u, G = part ? share : 1u;
+                    const uint32_t k_end = nst * (g + 1u) / G;
+                    // 64 records per round, two per lane, listed in staging
+                    // order
+                    for (uint32_t base = nst * g / G; base < k_end; base += 64) {
+                        unsigned bf[2], bw[2];
+                        bool fl[2], wa[2];
 #pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            fl[u] = (m[u] & omask) != 0u;
-                            wa[u] = (m[u] & wmask) != 0u;
-                            const unsigned bf = __ballot_sync(0xffffffffu, fl[u]);
-                            bw[u] = __ballot_sync(0xffffffffu, wa[u]);
-                            before += (uint32_t)__popc(bf & lt);
-                            tot += (uint32_t)__popc(bf);
-                            wtot |= bw[u];
+                        for (int v = 0; v < 2; v++) {
+                            const uint32_t k = base + 32u * v + lane;
+                            const float4 r = S.r0[min(k, (uint32_t)CAP)];
+                            const float dx = fmaxf(fmaxf(lo[0] - r.x, r.x - hi[0]), 0.f);
+                            const float dy = fmaxf(fmaxf(lo[1] - r.y, r.y - hi[1]), 0.f);
+                            const float dz = fmaxf(fmaxf(lo[2] - r.z, r.z - hi[2]), 0.f);
+                            const bool in = k < k_end && dx * dx + dy * dy + dz * dz < R2;
+                            fl[v] = in && r.w > 0.f;
+                            // the boundary elements matter to fluid only
+                            wa[v] = in && r.w < 0.f && any_fluid;
+                            bf[v] = __ballot_sync(0xffffffffu, fl[v]);
+                            bw[v] = __ballot_sync(0xffffffffu, wa[v]);
                         }
-                        {
-                            uint32_t p = fill + before;
-#pragma unroll
-                            for (int u = 0; u < 4; u++)
-                                if (fl[u])
-                                    list[p++] = (uint16_t)(k0 + u);
-                        }
-                        fill += tot;
+                        uint32_t wtot = bw[0] | bw[1], wbefore = 0;
+                        if (fl[0])
+                            list[fill + (uint32_t)__popc(bf[0] & lt)] = (uint16_t)(base + lane);
+                        fill += (uint32_t)__popc(bf[0]);
+                        if (fl[1])
+                            list[fill + (uint32_t)__popc(bf[1] & lt)] = (uint16_t)(base + 32u + lane);
+                        fill += (uint32_t)__popc(bf[1]);
                         if (wtot) {
-#pragma unroll
-                            for (int u = 0; u < 4; u++)
-                                wbefore += (uint32_t)__popc(bw[u] & lt);
-                            wtot = 0;
-#pragma unroll
-                            for (int u = 0; u < 4; u++)
-                                wtot += (uint32_t)__popc(bw[u]);
+                            wtot = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1]);
                             if (wfill + wtot > (uint32_t)kClWallCap) {
                                 // the wall list is full: sum it, and let the
                                 // epilogue walk the walls from global memory
@@ -967,14 +693,15 @@ k_sweep_cl(Consts c, StepArgs a)
                                 wdone = 0;
                                 walls_global = true;
                             }
-                            uint32_t q = wfill + wbefore;
-#pragma unroll
-                            for (int u = 0; u < 4; u++)
-                                if (wa[u])
-                                    wl[q++] = (uint16_t)(k0 + u);
+                            wbefore = (uint32_t)__popc(bw[0] & lt);
+                            if (wa[0])
+                                wl[wfill + wbefore] = (uint16_t)(base + lane);
+                            wbefore = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1] & lt);
+                            if (wa[1])
+                                wl[wfill + wbefore] = (uint16_t)(base + 32u + lane);
                             wfill += wtot;
                         }
-                        if (fill > (uint32_t)(kClListCap - 128)) {
+                        if (fill > (uint32_t)(kClListCap - 64)) {
                             __syncwarp();
                             const uint32_t nq = fill / 4;
                             drain(list, nq, false);
@@ -1005,23 +732,46 @@ k_sweep_cl(Consts c, StepArgs a)
                 }
                 if (failed)
                     break;
-                if (have) {
-                    shep = shep + shep;  // the pair sums hold half of it
-                    // ---- the four partial sums of each particle
-                    float* acc[13] = { &shep, &gp0, &gp1, &gp2, &lu0, &lu1, &lu2,
-                                       &du, &lp, &gw0, &gw1, &gw2, &dbi };
+                // ---- the four partial sums of each particle
+                float* acc[kClSums] = { &shep, &gp0, &gp1, &gp2, &lu0, &lu1, &lu2,
+                                        &du, &lp, &gw0, &gw1, &gw2, &dbi };
+                if (combine) {
+                    // the parts of the cluster, in order
+                    walls_global = false;
+                    for (uint32_t k = 0; k < share; k++)
+                        walls_global = walls_global || (S.wn[warp * share + k] >> 31);
 #pragma unroll
-                    for (int k = 0; k < 13; k++) {
+                    for (int k = 0; k < kClSums; k++) {
+                        float v = S.part[warp * share][k][mq];
+                        for (uint32_t g = 1; g < share; g++)
+                            v = v + S.part[warp * share + g][k][mq];
+                        *acc[k] = v;
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kClSums; k++) {
                         float v = *acc[k];
                         v = v + __shfl_xor_sync(0xffffffffu, v, 8);
                         v = v + __shfl_xor_sync(0xffffffffu, v, 16);
                         *acc[k] = v;
                     }
-                    const float v = sweep_cl_finish(
+                    if (lane == 0)
+                        S.wn[warp] = wfill | (part && walls_global ? 0x80000000u : 0u);
+                }
+                if (part) {
+                    if (q == 0)
+#pragma unroll
+                        for (int k = 0; k < kClSums; k++)
+                            S.part[u][k][mq] = *acc[k];
+                } else if (have) {
+                    __syncwarp();
+                    shep = shep + shep;  // the pair sums hold half of it
+                    const float v = sweep_cl_finish<NW, CAP>(
                         c, a, i, valid, im, want, fluid, sensor, q == 0, dt,
                         r0i, r1i, shep, gp0, gp1, gp2, lu0, lu1, lu2, du, lp,
-                        gw0, gw1, gw2, dbi, walls_global, wl, wfill, S.r0,
-                        S.r1, key, cas);
+                        gw0, gw1, gw2, dbi, walls_global, S,
+                        combine ? warp * share : (uint32_t)warp,
+                        combine ? share : 1u, key, cas);
                     float vm = v;
                     for (int o = 16; o > 0; o >>= 1)
                         vm = cl_min(vm, __shfl_xor_sync(0xffffffffu, vm, o));
@@ -1032,10 +782,10 @@ k_sweep_cl(Consts c, StepArgs a)
                     }
                     run_min = cl_min(run_min, vm);
                 }
-                if (!single)
-                    break;  // one cluster per warp per wave
                 __syncwarp();
             }
+            if (combine)
+                break;
         }
         if (failed)
             break;

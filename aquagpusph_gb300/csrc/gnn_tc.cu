@@ -30,6 +30,14 @@ constexpr int kTcThreads = 128;
 constexpr int kTcRows = 128;
 constexpr uint32_t kWaitLimit = 1u << 22;
 
+// bytes of a 128 x K operand tile that the epilogue reuses: 4 KB per warp
+inline size_t
+tc_operand_bytes(uint32_t K)
+{
+    const size_t tile = (size_t)kTcRows * K * 2, out = (size_t)kTcThreads / 32 * 4096;
+    return tile > out ? tile : out;
+}
+
 __device__ __forceinline__ uint32_t
 smem_addr(const void* p)
 {
@@ -81,23 +89,104 @@ pack2(float lo, float hi)
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// copy a rows x K bf16 block (row-major, ld elements) into the core-matrix
-// layout: element (r, k) at ((r / 8) * (K / 8) + k / 8) * 128 + (r % 8) * 16
-// + (k % 8) * 2 bytes; rows past `valid` are zero
+// Starts asynchronous copies of a rows x K bf16 block (row-major, ld elements,
+// rows a multiple of 8, K of 16) into core matrices of 8 rows x 16 bytes:
+// element (r, k) goes to (r / 8) * row_step + (k / 8) * col_step + (r % 8) * 16
+// + (k % 8) * 2; rows past `valid` are filled with zeros.  Eight consecutive
+// lanes fill one core matrix (128 contiguous bytes, no bank conflict) and
+// sixteen read whole 32-byte sectors of eight rows.
+__device__ __forceinline__ void
+stage_async(uint8_t* dst, const uint16_t* src, uint32_t ld, uint32_t rows,
+            uint32_t valid, uint32_t K, uint32_t row_step, uint32_t col_step)
+{
+    const uint32_t r8 = threadIdx.x & 7, h = (threadIdx.x >> 3) & 1;
+    const uint32_t pairs = K / 16, tasks = rows / 8 * pairs;
+    const uint32_t step = blockDim.x / 16;
+    // (row block, pair of column groups) of this half-warp's next task
+    uint32_t rb = (threadIdx.x >> 4) / pairs, pr = (threadIdx.x >> 4) % pairs;
+    const uint32_t drb = step / pairs, dpr = step % pairs;
+    for (uint32_t t = threadIdx.x >> 4; t < tasks; t += step) {
+        const uint32_t g = pr * 2 + h;
+        const uint32_t r = rb * 8 + r8;
+        const bool ok = r < valid;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                     :: "r"(smem_addr(dst + rb * row_step + g * col_step + r8 * 16)),
+                        "l"(src + (size_t)(ok ? r : 0u) * ld + g * 8), "r"(ok ? 16u : 0u)
+                     : "memory");
+        rb += drb;
+        pr += dpr;
+        if (pr >= pairs) {
+            pr -= pairs;
+            rb++;
+        }
+    }
+}
+
+__device__ __forceinline__ void
+stage_wait()
+{
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+// K-major operand: rows x K with consecutive core matrices along K
 __device__ __forceinline__ void
 stage(uint8_t* dst, const uint16_t* src, uint32_t ld, uint32_t rows,
       uint32_t valid, uint32_t K)
 {
-    const uint32_t kg = K / 8;
-    for (uint32_t e = threadIdx.x; e < rows * kg; e += kTcThreads) {
-        const uint32_t r = e / kg, g = e % kg;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < valid)
-            v = *reinterpret_cast<const uint4*>(src + (size_t)r * ld + g * 8);
-        *reinterpret_cast<uint4*>(dst + ((r / 8) * kg + g) * 128 + (r % 8) * 16) = v;
-    }
+    stage_async(dst, src, ld, rows, valid, K, K / 8 * 128, 128);
+    stage_wait();
 }
 
+// One warp's 32 rows x 128 bytes in shared memory, 16-byte chunk c of row r
+// at chunk c ^ (r % 8): a lane writes or reads its own row, or a warp whole
+// rows of global memory (4 per instruction), either way without bank
+// conflicts.  Rows of 64 bytes (32 bf16) use chunks 0-3 in the same way.
+__device__ __forceinline__ uint4*
+warp_chunk(uint8_t* buf, uint32_t r, uint32_t c)
+{
+    return reinterpret_cast<uint4*>(buf + r * 128 + ((c ^ (r & 7)) * 16));
+}
+
+// Copies `chunks` (2, 4 or 8) 16-byte chunks of each of the warp's rows to
+// global memory: row r at g + r * ld bytes, r < valid
+__device__ __forceinline__ void
+warp_store_rows(uint8_t* buf, uint8_t* g, size_t ld, uint32_t valid,
+                uint32_t chunks)
+{
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t per = 32 / chunks, c = lane % chunks;
+    for (uint32_t r = lane / chunks; r < 32; r += per)
+        if (r < valid)
+            *reinterpret_cast<uint4*>(g + r * ld + c * 16) = *warp_chunk(buf, r, c);
+}
+
+// 32 columns of the warp's 32 tensor-memory lanes
+__device__ __forceinline__ void
+ld_tmem32(uint32_t addr, float (&z)[32])
+{
+    uint32_t v[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
+          "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
+          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
+          "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
+          "=r"(v[31])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n");
+#pragma unroll
+    for (int j = 0; j < 32; j++)
+        z[j] = __uint_as_float(v[j]);
+}
+
+// Bound by memory: a row of 64 inputs with both outputs moves 512 bytes.
+// Rows leave through shared memory (stores of whole rows): with each lane
+// storing 16 bytes of its own row the load / store unit was 72% busy and
+// 10.3M rows took 1.82 ms; now 0.90.
 template<int N>
 __global__ void __launch_bounds__(kTcThreads, 1)
 k_linear_fwd_tc(uint32_t M, uint32_t K, const uint16_t* __restrict__ X,
@@ -108,9 +197,13 @@ k_linear_fwd_tc(uint32_t M, uint32_t K, const uint16_t* __restrict__ X,
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float sbias[N];
     uint8_t* sB = smem;                                // N x K
-    uint8_t* sA = smem + ((N * K * 2 + 1023) / 1024) * 1024;  // 128 x K
+    // 128 x K, and 4 KB per warp for the outputs
+    uint8_t* sA = smem + ((N * K * 2 + 1023) / 1024) * 1024;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x < N)
+        sbias[threadIdx.x] = bias ? bias[threadIdx.x] : 0.f;
 
     stage(sB, W, K, N, N, K);
     if (threadIdx.x == 0) {
@@ -173,39 +266,47 @@ k_linear_fwd_tc(uint32_t M, uint32_t K, const uint16_t* __restrict__ X,
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;\n");
         // epilogue: warp w owns rows 32w .. 32w + 31 (TMEM lanes)
-        const uint32_t row = m0 + warp * 32 + lane;
+        // 32 columns at a time, through the warp's rows of the operand buffer
+        // (its MMAs have completed) so that they leave as whole rows
+        const uint32_t row0 = m0 + warp * 32;
+        const uint32_t wvalid = row0 < M ? min(32u, M - row0) : 0u;
         const uint32_t taddr = tmem + ((warp * 32u) << 16);
+        uint8_t* wbuf = sA + warp * 4096;
 #pragma unroll
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            uint32_t v[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]),
-                  "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                  "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                  "=r"(v[14]), "=r"(v[15])
-                : "r"(taddr + (uint32_t)c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n");
-            if (row < M) {
-                float z[16];
-                for (int j = 0; j < 16; j++)
-                    z[j] = __uint_as_float(v[j]) + (bias ? bias[c0 + j] : 0.f);
-                if (Z)
-                    for (int j = 0; j < 16; j += 4)
-                        *reinterpret_cast<float4*>(Z + (size_t)row * ldz + c0 + j) =
-                            make_float4(z[j], z[j + 1], z[j + 2], z[j + 3]);
-                if (Y) {
-                    uint32_t p[8];
-                    for (int j = 0; j < 8; j++) {
-                        p[j] = pack2(z[2 * j], z[2 * j + 1]);
-                        if (act == AQUA_ACT_SILU)
-                            p[j] = silu_bf16x2(p[j]);
-                    }
-                    uint4* dst = reinterpret_cast<uint4*>(Y + (size_t)row * ldy + c0);
-                    dst[0] = make_uint4(p[0], p[1], p[2], p[3]);
-                    dst[1] = make_uint4(p[4], p[5], p[6], p[7]);
+        for (int c0 = 0; c0 < N; c0 += 32) {
+            float z[32];
+            ld_tmem32(taddr + (uint32_t)c0, z);
+            if (bias)
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 b4 = *reinterpret_cast<const float4*>(sbias + c0 + j);
+                    z[j] += b4.x;
+                    z[j + 1] += b4.y;
+                    z[j + 2] += b4.z;
+                    z[j + 3] += b4.w;
                 }
+            if (Z) {
+                __syncwarp();
+                for (int j = 0; j < 8; j++)
+                    *reinterpret_cast<float4*>(warp_chunk(wbuf, lane, j)) =
+                        make_float4(z[4 * j], z[4 * j + 1], z[4 * j + 2], z[4 * j + 3]);
+                __syncwarp();
+                warp_store_rows(wbuf, reinterpret_cast<uint8_t*>(Z + (size_t)row0 * ldz + c0),
+                                (size_t)ldz * 4, wvalid, 8);
+            }
+            if (Y) {
+                uint32_t p[16];
+                for (int j = 0; j < 16; j++) {
+                    p[j] = pack2(z[2 * j], z[2 * j + 1]);
+                    if (act == AQUA_ACT_SILU)
+                        p[j] = silu_bf16x2(p[j]);
+                }
+                __syncwarp();
+                for (int j = 0; j < 4; j++)
+                    *warp_chunk(wbuf, lane, j) =
+                        make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2], p[4 * j + 3]);
+                __syncwarp();
+                warp_store_rows(wbuf, reinterpret_cast<uint8_t*>(Y + (size_t)row0 * ldy + c0),
+                                (size_t)ldy * 2, wvalid, 4);
             }
         }
         // the next tile's MMAs overwrite the accumulator and sA
@@ -699,7 +800,15 @@ static_assert(edge_ctas_per_sm<false>() * (edge_mlp_smem<80>() + 1024) <= 228 * 
 __device__ __forceinline__ float
 silu_grad_f(float z)
 {
-    const float s = 1.f / (1.f + __expf(-z));
+    // 1 / b by two Newton steps, free of branches up to b = 2^100: the IEEE
+    // reciprocal but for about one value in 5e7 (one ulp)
+    const float b = 1.f + __expf(-z);
+    float s;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(b));
+    s = __fmaf_rn(s, __fmaf_rn(-b, s, 1.f), s);
+    s = __fmaf_rn(s, __fmaf_rn(-b, s, 1.f), s);
+    if (b > 0x1p100f)
+        s = 1.f / b;
     return s * (1.f + z * (1.f - s));
 }
 
@@ -731,7 +840,8 @@ k_linear_dgrad_tc(uint32_t M, uint32_t N, uint32_t K,
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base;
     uint8_t* sB = smem;                                        // K x N
-    uint8_t* sA = smem + ((K * N * 2 + 1023) / 1024) * 1024;   // 128 x N
+    // 128 x N, and 4 KB per warp for Zp and dX
+    uint8_t* sA = smem + ((K * N * 2 + 1023) / 1024) * 1024;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     stage(sB, Wt, N, K, K, N);
@@ -749,6 +859,7 @@ k_linear_dgrad_tc(uint32_t M, uint32_t N, uint32_t K,
     const uint32_t tmem = tmem_base;
     const uint32_t idesc = make_idesc(K);
     const uint32_t sbo = (N / 8) * 128;
+    const bool grad = Zp && act_prev == AQUA_ACT_SILU;
     uint32_t phase = 0;
     const uint32_t tiles = (M + kTcRows - 1) / kTcRows;
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -779,41 +890,77 @@ k_linear_dgrad_tc(uint32_t M, uint32_t N, uint32_t K,
         }
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;\n");
-        // epilogue: warp w owns rows 32w .. 32w + 31 (TMEM lanes)
-        const uint32_t row = m0 + warp * 32 + lane;
+        // epilogue: warp w owns rows 32w .. 32w + 31 (TMEM lanes), 32 columns
+        // at a time (the last 16 alone); Zp and dX pass through the warp's
+        // rows of the operand buffer so that whole rows move
+        const uint32_t row0 = m0 + warp * 32;
+        const uint32_t wvalid = row0 < M ? min(32u, M - row0) : 0u;
         const uint32_t taddr = tmem + ((warp * 32u) << 16);
-        for (uint32_t c0 = 0; c0 < K; c0 += 16) {
-            uint32_t v[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]),
-                  "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                  "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-                  "=r"(v[14]), "=r"(v[15])
-                : "r"(taddr + c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n");
-            if (row < M) {
+        uint8_t* wbuf = sA + warp * 4096;
+        for (uint32_t c0 = 0; c0 < K; c0 += 32) {
+            const uint32_t w16 = min(32u, K - c0) / 16u;  // 16-column groups
+            if (grad) {
+                // rows of Zp -> shared memory (8 chunks of 4 floats, or 4)
+                const uint32_t ch = 4u * w16, per = 32u / ch, cc = lane % ch;
+                const float* zp = Zp + (size_t)row0 * ldzp + c0;
+                float4 zz[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const uint32_t r = lane / ch + q * per;
+                    zz[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (r < wvalid && r < 32u)
+                        zz[q] = *reinterpret_cast<const float4*>(zp + (size_t)r * ldzp + cc * 4);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const uint32_t r = lane / ch + q * per;
+                    if (r < 32u)
+                        *reinterpret_cast<float4*>(warp_chunk(wbuf, r, cc)) = zz[q];
+                }
+                __syncwarp();
+            }
+            uint32_t pk[16];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (h >= (int)w16)
+                    break;
+                uint32_t v[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]),
+                      "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                      "=r"(v[14]), "=r"(v[15])
+                    : "r"(taddr + c0 + 16 * h));
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n");
                 float d[16];
                 for (int j = 0; j < 16; j++)
                     d[j] = __uint_as_float(v[j]);
-                if (Zp && act_prev == AQUA_ACT_SILU) {
-                    const float* z = Zp + (size_t)row * ldzp + c0;
+                if (grad) {
                     for (int j = 0; j < 16; j += 4) {
-                        const float4 zz = *reinterpret_cast<const float4*>(z + j);
+                        const float4 zz = *reinterpret_cast<const float4*>(
+                            warp_chunk(wbuf, lane, 4 * h + j / 4));
                         d[j] *= silu_grad_f(zz.x);
                         d[j + 1] *= silu_grad_f(zz.y);
                         d[j + 2] *= silu_grad_f(zz.z);
                         d[j + 3] *= silu_grad_f(zz.w);
                     }
                 }
-                uint32_t pk[8];
                 for (int j = 0; j < 8; j++)
-                    pk[j] = pack2(d[2 * j], d[2 * j + 1]);
-                uint4* dst = reinterpret_cast<uint4*>(dX + (size_t)row * ldx + c0);
-                dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                    pk[8 * h + j] = pack2(d[2 * j], d[2 * j + 1]);
             }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (j < 2 * (int)w16)
+                    *warp_chunk(wbuf, lane, j) =
+                        make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+            __syncwarp();
+            warp_store_rows(wbuf, reinterpret_cast<uint8_t*>(dX + (size_t)row0 * ldx + c0),
+                            (size_t)ldx * 2, wvalid, 2u * w16);
+            __syncwarp();
         }
         // the next tile's MMAs overwrite the accumulator and sA
         asm volatile("tcgen05.fence::before_thread_sync;\n");
@@ -824,42 +971,6 @@ k_linear_dgrad_tc(uint32_t M, uint32_t N, uint32_t K,
         asm volatile("tcgen05.fence::after_thread_sync;\n");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n"
                      :: "r"(tmem), "r"(tcols));
-    }
-}
-
-// rows x 128 transposed block: element (r, m) = src[m * ld + r] for r < nr
-// and m < valid (zero for m >= valid), into the core-matrix layout with 128
-// reduction columns (16 core matrices per 8-row group); rows >= nr are left
-// as they are.  Each warp task moves four 8 x 8 blocks (four consecutive
-// 8-row groups of m, one 8-column group of r): every lane loads its
-// fragment element pair from global memory (row m = lane / 4, columns
-// 2 (lane % 4) and the next) and stmatrix .trans writes each block
-// transposed, whole 16-byte rows of a core matrix, free of bank conflicts.
-__device__ __forceinline__ void
-stage_t(uint8_t* dst, const uint16_t* src, uint32_t ld, uint32_t nr,
-        uint32_t valid)
-{
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rg = nr / 8;                        // 8-column groups of r
-    const uint32_t ar = lane >> 2, ac = (lane & 3) * 2;  // fragment position
-    const uint32_t mi = lane >> 3, mj = lane & 7;        // row address role
-    for (uint32_t t = warp; t < 4 * rg; t += blockDim.x / 32) {
-        const uint32_t mg = t & 3, kb = t >> 2;
-        uint32_t v[4];
-        for (int i = 0; i < 4; i++) {
-            const uint32_t m = (mg * 4 + i) * 8 + ar;
-            v[i] = m < valid ? *reinterpret_cast<const uint32_t*>(
-                                   src + (size_t)m * ld + kb * 8 + ac)
-                             : 0u;
-        }
-        // lane 8i + j: row j of block i, stored transposed at the core
-        // matrix (r group kb, m group 4 mg + i)
-        const uint32_t addr =
-            smem_addr(dst + (kb * 16 + mg * 4 + mi) * 128 + mj * 16);
-        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 "
-                     "[%0], {%1, %2, %3, %4};\n"
-                     :: "r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
-                     : "memory");
     }
 }
 
@@ -876,8 +987,12 @@ k_linear_wgrad_tc(uint32_t M, uint32_t N, uint32_t K,
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_base;
     // nbuf (1 or 2) buffers, each A = dY^T (128 rows, N used) x 128 and
-    // B = X^T (KB rows: X^T, then the row of ones for db, then zeros) x 128;
-    // with two, a chunk is staged while the MMAs of the previous one run
+    // B = X^T (KB rows: X^T, then the row of ones for db, then zeros) x 128,
+    // both MN-major: core matrices of 8 reduction rows x 16 bytes, as the
+    // rows lie in memory (no transposition: 10.3M rows with the 4-byte loads
+    // and stmatrix.trans of one took 1.08 ms, now 0.80); 16 core matrices
+    // along the reduction per 8 outputs.  With two buffers a chunk is copied
+    // while the MMAs of the one before run.
     const uint32_t bufb = 128 * 128 * 2 + KB * 128 * 2;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t chunks = (M + kTcRows - 1) / kTcRows;
@@ -892,7 +1007,7 @@ k_linear_wgrad_tc(uint32_t M, uint32_t N, uint32_t K,
             const uint32_t r = K + e / 128u, m = e % 128u;
             const uint16_t one = (r == K && db) ? 0x3F80u : 0u;  // bf16 1.0
             *reinterpret_cast<uint16_t*>(
-                sB + ((r / 8) * 16 + m / 8) * 128 + (r % 8) * 16 + (m % 8) * 2) = one;
+                sB + ((r / 8) * 16 + m / 8) * 128 + (m % 8) * 16 + (r % 8) * 2) = one;
         }
     }
     if (threadIdx.x == 0)
@@ -908,29 +1023,59 @@ k_linear_wgrad_tc(uint32_t M, uint32_t N, uint32_t K,
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     const uint32_t tmem = tmem_base;
-    const uint32_t idesc = make_idesc(KB);
-    constexpr uint32_t sbo = 16 * 128;  // 128 reduction columns per row group
+    // A and B MN-major (bits 15, 16)
+    const uint32_t idesc = make_idesc(KB) | (1u << 15) | (1u << 16);
+    constexpr uint32_t sbo = 16 * 128;  // next 8 outputs: 16 core matrices on
     uint32_t phase[2] = { 0u, 0u };
     uint32_t pending[2] = { 0u, 0u };  // a commit of the buffer not yet waited
     bool failed = false;
     uint32_t it = 0;
+    // starts the copies of a chunk into buffer b, one group
+    auto copy = [&](uint32_t ch, uint32_t b) {
+        uint8_t* sA = smem + b * bufb;
+        uint8_t* sB = sA + 128 * 128 * 2;
+        const uint32_t m0 = ch * kTcRows;
+        const uint32_t valid = min((uint32_t)kTcRows, M - m0);
+        stage_async(sA, dY + (size_t)m0 * ldy, ldy, kTcRows, valid, N, 128, 16 * 128);
+        stage_async(sB, X + (size_t)m0 * ldx, ldx, kTcRows, valid, K, 128, 16 * 128);
+    };
+    // waits for the MMAs that read buffer b
+    auto drained = [&](uint32_t b) -> bool {
+        if (!pending[b])
+            return true;
+        if (!tc_wait(&mbar[b], phase[b], fake))
+            return false;
+        phase[b] ^= 1u;
+        pending[b] = 0u;
+        return true;
+    };
+    if (nbuf == 2) {
+        copy(blockIdx.x, 0);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
     for (uint32_t ch = blockIdx.x; ch < chunks && !failed; ch += gridDim.x, it++) {
         const uint32_t b = it % nbuf;
         uint8_t* sA = smem + b * bufb;
         uint8_t* sB = sA + 128 * 128 * 2;
-        // the MMAs of the chunk nbuf ago read this buffer
-        if (pending[b]) {
-            if (!tc_wait(&mbar[b], phase[b], fake)) {
+        if (nbuf == 2) {
+            // the next chunk into the other buffer, then wait for this one's
+            if (ch + gridDim.x < chunks) {
+                if (!drained(b ^ 1u)) {
+                    failed = true;
+                    break;
+                }
+                copy(ch + gridDim.x, b ^ 1u);
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        } else {
+            if (!drained(b)) {
                 failed = true;
                 break;
             }
-            phase[b] ^= 1u;
-            pending[b] = 0u;
+            copy(ch, b);
+            stage_wait();
         }
-        const uint32_t m0 = ch * kTcRows;
-        const uint32_t valid = min((uint32_t)kTcRows, M - m0);
-        stage_t(sA, dY + (size_t)m0 * ldy, ldy, N, valid);
-        stage_t(sB, X + (size_t)m0 * ldx, ldx, K, valid);
         asm volatile("fence.proxy.async.shared::cta;\n");
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -949,6 +1094,7 @@ k_linear_wgrad_tc(uint32_t M, uint32_t N, uint32_t K,
         }
         pending[b] = 1u;
     }
+    stage_wait();  // none is left in flight
     // the last commits (the MMAs run in order: the later one covers both)
     for (int b = 0; b < 2; b++) {
         if (!pending[b])
@@ -1169,8 +1315,7 @@ aqua_gnn_linear_fwd_tc(uint32_t M, uint32_t K, uint32_t N, const uint16_t* X,
         return AQUA_ERR_INVALID;
     if (M == 0)
         return AQUA_OK;
-    size_t bytes = ((size_t)N * K * 2 + 1023) / 1024 * 1024 +
-                   (size_t)kTcRows * K * 2;
+    size_t bytes = ((size_t)N * K * 2 + 1023) / 1024 * 1024 + tc_operand_bytes(K);
     // at least 30 KB per CTA keeps <= 7 CTAs on an SM (7 x 64 of the 512
     // tensor-memory columns), so tcgen05.alloc never has to wait
     if (bytes < 30 * 1024)
@@ -1249,7 +1394,7 @@ aqua_gnn_linear_dgrad_tc(uint32_t M, uint32_t N, uint32_t K,
     if (M == 0)
         return AQUA_OK;
     const uint32_t tcols = tc_cols(K);
-    size_t bytes = ((size_t)K * N * 2 + 1023) / 1024 * 1024 + (size_t)kTcRows * N * 2;
+    size_t bytes = ((size_t)K * N * 2 + 1023) / 1024 * 1024 + tc_operand_bytes(N);
     if (bytes < tc_min_smem(tcols))
         bytes = tc_min_smem(tcols);
     int sms = 0;

@@ -72,6 +72,7 @@ struct aqua_ctx
     static constexpr int kStageRing = 4;
     uint8_t* stage[2][kStageRing] = {};
     cudaEvent_t stage_ev[2][kStageRing] = {};
+    uint8_t* aux = nullptr;        // pinned: the scalars aqua_linklist() returns
     int stage_next[2] = { 0, 0 };  // the ring entry stage_begin hands out
     int stage_cur[2] = { 0, 0 };   // the entry in use, for stage_done
     // stage boundary events (recorded when profiling is on): before the
@@ -332,7 +333,7 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
         AQ_CUDA(cudaEventRecordWithFlags(x->ev[0], s, cudaEventRecordExternal));
     AQ_CUDA(launch_begin(x->sc, x->cs, x->n_cases, b.cells, b.wall_range,
                          x->consts.sample_on ? b.cell_mark : nullptr, x->ncap,
-                         N, s));
+                         N, b.sort_scratch, s));
     // one case: every particle's case id is 0 (not read)
     const uint32_t* cid = x->n_cases > 1 ? S.cid : nullptr;
     if (x->dims == 3) {
@@ -575,6 +576,7 @@ aqua_create(const aqua_params* params, uint32_t capacity,
             ok = cudaMallocHost(&x->stage[k][q], kStageBytes) == cudaSuccess &&
                  cudaEventCreateWithFlags(&x->stage_ev[k][q],
                                           cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && cudaMallocHost(&x->aux, kStageCs + sizeof(CaseScalars)) == cudaSuccess;
     if (!ok) {
         aqua_destroy(x);
         return AQUA_ERR_CUDA;
@@ -603,6 +605,8 @@ aqua_destroy(aqua_ctx* x)
             if (x->stage[k][q])
                 cudaFreeHost(x->stage[k][q]);
         }
+    if (x->aux)
+        cudaFreeHost(x->aux);
     if (x->pool)
         cudaFree(x->pool);
     delete x;
@@ -1037,11 +1041,9 @@ aqua_linklist(aqua_ctx* x, const float* r_in, uint32_t N, uint32_t* icell,
     StepBufs& b = x->b;
     const uint32_t ncap = ihoc_capacity < x->ncap ? ihoc_capacity : x->ncap;
     const uint32_t passes = sort_passes(bits_for(ncap));
-    DevScalars hs;
-    std::memset(&hs, 0, sizeof(hs));
-    AQ_CUDA(cudaMemcpyAsync(x->sc_aux, &hs, sizeof(hs), cudaMemcpyHostToDevice, s));
+    AQ_CUDA(cudaMemsetAsync(x->sc_aux, 0, sizeof(DevScalars), s));
     AQ_CUDA(launch_begin(x->sc_aux, x->cs_aux, 1, b.cells, b.wall_range,
-                         nullptr, 0, N, s));
+                         nullptr, 0, N, b.sort_scratch, s));
     if (x->dims == 3) {
         AQ_CUDA(launch_minmax<3>(x->consts, r_in, nullptr, nullptr, N, x->cs_aux,
                                  x->sc_aux, s));
@@ -1057,20 +1059,19 @@ aqua_linklist(aqua_ctx* x, const float* r_in, uint32_t N, uint32_t* icell,
                                      x->cs_aux, x->sc_aux, b.keys[0],
                                      b.sort_scratch, passes, s));
     }
+    // the last pass writes the caller's buffers
     AQ_CUDA(launch_radix_passes(b.keys, b.vals, N, passes, b.sort_scratch,
-                                true, x->sc_aux, s));
-    const int r = passes & 1;
-    AQ_CUDA(cudaMemcpyAsync(icell, b.keys[r], N * 4ull, cudaMemcpyDeviceToDevice, s));
-    if (id_unsorted)
-        AQ_CUDA(cudaMemcpyAsync(id_unsorted, b.vals[r], N * 4ull,
-                                cudaMemcpyDeviceToDevice, s));
-    if (id_sorted)
-        AQ_CUDA(launch_inverse_perm(b.vals[r], id_sorted, N, x->sc_aux, s));
-    AQ_CUDA(launch_ihoc(b.keys[r], N, ihoc, ncap, x->sc_aux, s));
-    CaseScalars hc;
-    AQ_CUDA(cudaMemcpyAsync(&hs, x->sc_aux, sizeof(hs), cudaMemcpyDeviceToHost, s));
-    AQ_CUDA(cudaMemcpyAsync(&hc, x->cs_aux, sizeof(hc), cudaMemcpyDeviceToHost, s));
+                                true, x->sc_aux, s, icell, id_unsorted,
+                                id_sorted));
+    AQ_CUDA(launch_ihoc(icell, N, ihoc, ncap, x->sc_aux, s));
+    // the scalars through pinned memory (a copy to pageable memory waits for
+    // the device by itself, one after the other)
+    AQ_CUDA(cudaMemcpyAsync(x->aux, x->sc_aux, sizeof(DevScalars), cudaMemcpyDeviceToHost, s));
+    AQ_CUDA(cudaMemcpyAsync(x->aux + kStageCs, x->cs_aux, sizeof(CaseScalars),
+                            cudaMemcpyDeviceToHost, s));
     AQ_CUDA(cudaStreamSynchronize(s));
+    const DevScalars hs = *reinterpret_cast<const DevScalars*>(x->aux);
+    const CaseScalars& hc = *reinterpret_cast<const CaseScalars*>(x->aux + kStageCs);
     if (n_cells_host)
         std::memcpy(n_cells_host, hc.n_cells, sizeof(hc.n_cells));
     if (r_min_host)
@@ -1078,8 +1079,7 @@ aqua_linklist(aqua_ctx* x, const float* r_in, uint32_t N, uint32_t* icell,
     if (r_max_host)
         std::memcpy(r_max_host, hc.r_max, sizeof(hc.r_max));
     if (hs.err) {
-        const uint32_t zero = 0;
-        AQ_CUDA(cudaMemcpyAsync(&x->sc_aux->err, &zero, 4, cudaMemcpyHostToDevice, s));
+        AQ_CUDA(cudaMemsetAsync(&x->sc_aux->err, 0, 4, s));
         AQ_CUDA(cudaStreamSynchronize(s));
     }
     return status_of(hs.err);

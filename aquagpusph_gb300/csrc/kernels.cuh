@@ -91,7 +91,8 @@ struct Vec<2>
 // may be NULL: every particle then belongs to case 0.
 cudaError_t launch_begin(DevScalars* sc, CaseScalars* cs, uint32_t n_cases,
                          uint2* cells, uint2* wall_range, uint8_t* cell_mark,
-                         uint32_t ncap, uint32_t N, cudaStream_t s);
+                         uint32_t ncap, uint32_t N, uint32_t* sort_scratch,
+                         cudaStream_t s);
 template<int D>
 cudaError_t launch_minmax(const Consts& c, const float* r, const int32_t* imove,
                           const uint32_t* cid, uint32_t N, CaseScalars* cs,
@@ -99,8 +100,8 @@ cudaError_t launch_minmax(const Consts& c, const float* r, const int32_t* imove,
 template<int D>
 cudaError_t launch_ncells(const Consts& c, CaseScalars* cs, uint32_t n_cases,
                           DevScalars* sc, uint32_t ncap, cudaStream_t s);
-// icell keys of the positions and the digit histograms (resets the sort
-// scratch first); then launch_radix_passes(..., hist_ready = true)
+// icell keys of the positions and the digit histograms (launch_begin() has
+// reset the sort scratch); then launch_radix_passes(..., hist_ready = true)
 template<int D>
 cudaError_t launch_icell_hist(const Consts& c, const float* r,
                               const int32_t* imove, const uint32_t* cid,
@@ -110,7 +111,9 @@ cudaError_t launch_icell_hist(const Consts& c, const float* r,
 cudaError_t launch_radix_passes(uint32_t* keys[2], uint32_t* vals[2],
                                 uint32_t n, uint32_t passes, uint32_t* scratch,
                                 bool hist_ready, DevScalars* sc,
-                                cudaStream_t s);
+                                cudaStream_t s, uint32_t* last_keys = nullptr,
+                                uint32_t* last_vals = nullptr,
+                                uint32_t* inverse = nullptr);
 size_t sort_scratch_words(uint32_t n);
 cudaError_t launch_inverse_perm(const uint32_t* perm, uint32_t* inv,
                                 uint32_t n, const DevScalars* sc,

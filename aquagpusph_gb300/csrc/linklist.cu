@@ -83,10 +83,12 @@ domain_position(const Consts& c, const float* r, const int32_t* imove,
         out[k] = x[k];
 }
 
-// Resets the per-step scalars of every case and clears the cell table.
+// Resets the per-step scalars of every case and clears the cell table and the
+// sort scratch (histograms, tile counters, the first pass's status array).
 __global__ void
 k_begin(DevScalars* sc, CaseScalars* cs, uint32_t n_cases, uint2* cells,
-        uint2* wall_range, uint8_t* cell_mark, uint32_t ncap, uint32_t N)
+        uint2* wall_range, uint8_t* cell_mark, uint32_t ncap, uint32_t N,
+        uint32_t* sort_scratch, uint32_t sort_words)
 {
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t k = tid; k < n_cases; k += gridDim.x * blockDim.x) {
@@ -102,6 +104,8 @@ k_begin(DevScalars* sc, CaseScalars* cs, uint32_t n_cases, uint2* cells,
     }
     if (sc->err)
         return;
+    for (uint32_t k = tid; k < sort_words; k += gridDim.x * blockDim.x)
+        sort_scratch[k] = 0;
     for (uint32_t c = tid; c < ncap; c += gridDim.x * blockDim.x) {
         cells[c] = make_uint2(N, N);
         wall_range[c] = make_uint2(0xffffffffu, 0u);
@@ -482,12 +486,13 @@ st_status(uint32_t* p, uint32_t v)
 // digit.  vals_in == nullptr stands for the identity (the first pass).
 // The pass also clears the other status array for the next pass.  A walk
 // that finds no status after kLookbackLimit polls records kErrTimeout and
-// goes on with what it has.
+// goes on with what it has.  The last pass may leave out the values and write
+// the inverse permutation.
 __global__ void __launch_bounds__(kSortThreads, 3)
 k_onesweep(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
            uint32_t* vals_out, uint32_t N, uint32_t shift,
            const uint32_t* ghist, uint32_t* counter, uint32_t* status,
-           uint32_t* status_next, DevScalars* sc)
+           uint32_t* status_next, DevScalars* sc, uint32_t* inverse)
 {
     __shared__ uint32_t s_keys[kSortTile];
     __shared__ uint32_t s_vals[kSortTile];
@@ -618,8 +623,12 @@ k_onesweep(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
     for (uint32_t q = t; q < nvalid; q += kSortThreads) {
         const uint32_t key = s_keys[q];
         const uint32_t g = s_gstart[(key >> shift) & 255u] + q;
+        const uint32_t val = s_vals[q];
         keys_out[g] = key;
-        vals_out[g] = s_vals[q];
+        if (vals_out)
+            vals_out[g] = val;
+        if (inverse)
+            inverse[val] = g;
     }
 }
 
@@ -678,11 +687,12 @@ grid_for(uint32_t n, unsigned threads)
 cudaError_t
 launch_begin(DevScalars* sc, CaseScalars* cs, uint32_t n_cases, uint2* cells,
              uint2* wall_range, uint8_t* cell_mark, uint32_t ncap, uint32_t N,
-             cudaStream_t s)
+             uint32_t* sort_scratch, cudaStream_t s)
 {
-    const unsigned g = min(grid_for(max(ncap, n_cases), 256), 152u * 8u);
+    const uint32_t words = kSortHdrWords + 256u * sort_blocks(N);
+    const unsigned g = min(grid_for(max(max(ncap, n_cases), words), 256), 152u * 8u);
     k_begin<<<max(g, 1u), 256, 0, s>>>(sc, cs, n_cases, cells, wall_range,
-                                        cell_mark, ncap, N);
+                                        cell_mark, ncap, N, sort_scratch, words);
     return cudaGetLastError();
 }
 
@@ -741,12 +751,15 @@ launch_sort_reset(uint32_t* scratch, uint32_t n, cudaStream_t s)
 }
 
 // Radix passes on the keys in keys[0] (values: the identity); the result
-// lands in keys/vals[passes & 1].  The scratch is reset here unless
-// `hist_ready` (the caller reset it and summed the histograms).
+// lands in keys/vals[passes & 1], or with `last_keys` in last_keys, last_vals
+// (may be NULL) and, the inverse permutation, `inverse` (may be NULL).  The
+// scratch is reset here unless `hist_ready` (the caller reset it and summed
+// the histograms).
 cudaError_t
 launch_radix_passes(uint32_t* keys[2], uint32_t* vals[2], uint32_t n,
                     uint32_t passes, uint32_t* scratch, bool hist_ready,
-                    DevScalars* sc, cudaStream_t s)
+                    DevScalars* sc, cudaStream_t s, uint32_t* last_keys,
+                    uint32_t* last_vals, uint32_t* inverse)
 {
     const uint32_t nb = sort_blocks(n);
     if (nb == 0)
@@ -766,10 +779,12 @@ launch_radix_passes(uint32_t* keys[2], uint32_t* vals[2], uint32_t n,
     }
     for (uint32_t p = 0; p < passes; p++) {
         const int in = p & 1, out = in ^ 1;
+        const bool last = p + 1 == passes && last_keys != nullptr;
         k_onesweep<<<nb, kSortThreads, 0, s>>>(
-            keys[in], p == 0 ? nullptr : vals[in], keys[out], vals[out], n,
-            8u * p, ghist + 256 * p, counters + p, stat[p & 1],
-            stat[(p + 1) & 1], sc);
+            keys[in], p == 0 ? nullptr : vals[in], last ? last_keys : keys[out],
+            last ? last_vals : vals[out], n, 8u * p, ghist + 256 * p,
+            counters + p, stat[p & 1], stat[(p + 1) & 1], sc,
+            last ? inverse : nullptr);
     }
     return cudaGetLastError();
 }
@@ -784,9 +799,6 @@ launch_icell_hist(const Consts& c, const float* r, const int32_t* imove,
     const uint32_t nb = sort_blocks(N);
     if (nb == 0)
         return cudaSuccess;
-    cudaError_t e = launch_sort_reset(scratch, N, s);
-    if (e != cudaSuccess)
-        return e;
     k_icell_hist<D><<<hist_grid(N), kSortThreads, 0, s>>>(
         c, r, imove, cid, N, cs, sc, keys, scratch, passes);
     return cudaGetLastError();

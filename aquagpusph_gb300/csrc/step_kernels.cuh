@@ -1244,10 +1244,8 @@ launch_bi_walls_impl(const Consts& c, const StepArgs& a, unsigned sms,
     if (a.N == 0)
         return cudaSuccess;
     const unsigned grid = sms * (16u / kQuadWarps);
-    if (a.cluster == 4)
-        k_bi_walls<D, 4><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
-    else
-        k_bi_walls<D, 8><<<grid, kQuadWarps * 32, 0, s>>>(c, a);
+    auto kernel = a.cluster == 4 ? k_bi_walls<D, 4> : k_bi_walls<D, 8>;
+    kernel<<<grid, kQuadWarps * 32, 0, s>>>(c, a);
     return cudaGetLastError();
 }
 

@@ -64,17 +64,17 @@ struct aqua_ctx
     // configuration the graphs were captured for (particles, cases, roll)
     uint32_t graph_n = 0, graph_cases = 0;
     int graph_motion = -1;
-    // pinned staging areas of the small host -> device copies (case scalars,
-    // motions, offsets): a ring of kStageRing for aqua_set_state and one for
-    // aqua_set_cases; an area is reused once its event shows that the copies
-    // that last read it executed, which with a ring of four is almost never
-    // a wait (the host may run several calls ahead of the device)
+    // pinned staging areas of aqua_set_cases' small host -> device copies
+    // (case scalars, motions, offsets), a ring of kStageRing: an area is
+    // reused once its event shows that the copies that last read it executed,
+    // which with a ring of four is almost never a wait (the host may run
+    // several calls ahead of the device)
     static constexpr int kStageRing = 4;
-    uint8_t* stage[2][kStageRing] = {};
-    cudaEvent_t stage_ev[2][kStageRing] = {};
+    uint8_t* stage[kStageRing] = {};
+    cudaEvent_t stage_ev[kStageRing] = {};
     uint8_t* aux = nullptr;        // pinned: the scalars aqua_linklist() returns
-    int stage_next[2] = { 0, 0 };  // the ring entry stage_begin hands out
-    int stage_cur[2] = { 0, 0 };   // the entry in use, for stage_done
+    int stage_next = 0;            // the ring entry stage_begin hands out
+    int stage_cur = 0;             // the entry in use, for stage_done
     // stage boundary events (recorded when profiling is on): before the
     // link-list, before the gather, before the sweep, after the sweep, end
     static constexpr int kEvents = 5;
@@ -285,28 +285,23 @@ constexpr size_t kStageCm = kStageCs + ((kMaxCases * sizeof(CaseScalars) + 255) 
 constexpr size_t kStageOff = kStageCm + ((kMaxCases * sizeof(CaseMotion) + 255) & ~(size_t)255);
 constexpr size_t kStageBytes = kStageOff + (kMaxCases + 1) * sizeof(uint32_t);
 
-// Staging area `slot` for the next small copies: waits (if at all) for the
-// copies that last read it, so that the host may overwrite it.  The copies
+// Staging area for the next small copies: waits (if at all) for the copies
+// that last read it, so that the host may overwrite it.  The copies
 // themselves stay asynchronous; stage_done() marks their position in the
 // stream.
-constexpr int kStageState = 0;  // aqua_set_state
-constexpr int kStageCases = 1;  // aqua_set_cases
-
 uint8_t*
-stage_begin(aqua_ctx* x, int slot)
+stage_begin(aqua_ctx* x)
 {
-    const int k = x->stage_next[slot];
-    x->stage_cur[slot] = k;
-    x->stage_next[slot] = (k + 1) % aqua_ctx::kStageRing;
-    return cudaEventSynchronize(x->stage_ev[slot][k]) == cudaSuccess
-               ? x->stage[slot][k]
-               : nullptr;
+    const int k = x->stage_next;
+    x->stage_cur = k;
+    x->stage_next = (k + 1) % aqua_ctx::kStageRing;
+    return cudaEventSynchronize(x->stage_ev[k]) == cudaSuccess ? x->stage[k] : nullptr;
 }
 
 cudaError_t
-stage_done(aqua_ctx* x, int slot, cudaStream_t s)
+stage_done(aqua_ctx* x, cudaStream_t s)
 {
-    return cudaEventRecord(x->stage_ev[slot][x->stage_cur[slot]], s);
+    return cudaEventRecord(x->stage_ev[x->stage_cur], s);
 }
 
 // The clustered sweep runs for the fast build in 3-D with BIe walls and the
@@ -426,14 +421,54 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
     return AQUA_OK;
 }
 
-aqua_status
-copy_in(void* dst, const void* src, size_t bytes, int on_host, cudaStream_t s)
+// Field copies of a state.  Between device arrays of this context's device,
+// one kernel copies all of them (and writes the records of `rec`); what it
+// must not touch (memory of another device or host, or not known to the
+// runtime, or not aligned to 4 bytes) goes by cudaMemcpyAsync, which takes
+// any address.  A field without source or destination is left out.
+struct Field
 {
-    if (!src)
-        return AQUA_ERR_INVALID;
-    AQ_CUDA(cudaMemcpyAsync(dst, src, bytes,
-                            on_host ? cudaMemcpyHostToDevice
-                                    : cudaMemcpyDeviceToDevice, s));
+    void* dst;
+    const void* src;
+    size_t bytes;
+};
+constexpr int kHostToDevice = 0, kDeviceToHost = 1, kOnDevice = 2;
+
+bool
+on_device(const aqua_ctx* x, const void* p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == x->device &&
+           (reinterpret_cast<uintptr_t>(p) & 3) == 0;
+}
+
+aqua_status
+copy_fields(aqua_ctx* x, const Field* f, size_t n, int kind,
+            const StateRecords& rec, cudaStream_t s)
+{
+    CopySpans sp;
+    sp.n = 0;
+    for (size_t k = 0; k < n; k++) {
+        if (!f[k].dst || !f[k].src)
+            continue;
+        // one end of each field is the context's own
+        const void* user = rec.cid ? f[k].src : f[k].dst;
+        if (kind == kOnDevice && sp.n < kMaxSpans && on_device(x, user)) {
+            sp.dst[sp.n] = static_cast<uint32_t*>(f[k].dst);
+            sp.src[sp.n] = static_cast<const uint32_t*>(f[k].src);
+            sp.words[sp.n++] = f[k].bytes / 4;
+            continue;
+        }
+        AQ_CUDA(cudaMemcpyAsync(f[k].dst, f[k].src, f[k].bytes,
+                                kind == kHostToDevice   ? cudaMemcpyHostToDevice
+                                : kind == kDeviceToHost ? cudaMemcpyDeviceToHost
+                                                        : cudaMemcpyDeviceToDevice, s));
+    }
+    AQ_CUDA(launch_copy_spans(sp, rec, s));
     return AQUA_OK;
 }
 
@@ -571,11 +606,10 @@ aqua_create(const aqua_params* params, uint32_t capacity,
     bool ok = cudaMemset(x->pool, 0, x->pool_bytes) == cudaSuccess &&
               cudaStreamCreateWithFlags(&x->cap_stream, cudaStreamNonBlocking) ==
                   cudaSuccess;
-    for (int k = 0; ok && k < 2; k++)
-        for (int q = 0; ok && q < aqua_ctx::kStageRing; q++)
-            ok = cudaMallocHost(&x->stage[k][q], kStageBytes) == cudaSuccess &&
-                 cudaEventCreateWithFlags(&x->stage_ev[k][q],
-                                          cudaEventDisableTiming) == cudaSuccess;
+    for (int q = 0; ok && q < aqua_ctx::kStageRing; q++)
+        ok = cudaMallocHost(&x->stage[q], kStageBytes) == cudaSuccess &&
+             cudaEventCreateWithFlags(&x->stage_ev[q], cudaEventDisableTiming) ==
+                 cudaSuccess;
     ok = ok && cudaMallocHost(&x->aux, kStageCs + sizeof(CaseScalars)) == cudaSuccess;
     if (!ok) {
         aqua_destroy(x);
@@ -596,15 +630,14 @@ aqua_destroy(aqua_ctx* x)
     for (int k = 0; k < aqua_ctx::kEvents; k++)
         if (x->ev[k])
             cudaEventDestroy(x->ev[k]);
-    for (int k = 0; k < 2; k++)
-        for (int q = 0; q < aqua_ctx::kStageRing; q++) {
-            if (x->stage_ev[k][q]) {
-                cudaEventSynchronize(x->stage_ev[k][q]);  // no copy still reads it
-                cudaEventDestroy(x->stage_ev[k][q]);
-            }
-            if (x->stage[k][q])
-                cudaFreeHost(x->stage[k][q]);
+    for (int q = 0; q < aqua_ctx::kStageRing; q++) {
+        if (x->stage_ev[q]) {
+            cudaEventSynchronize(x->stage_ev[q]);  // no copy still reads it
+            cudaEventDestroy(x->stage_ev[q]);
         }
+        if (x->stage[q])
+            cudaFreeHost(x->stage[q]);
+    }
     if (x->aux)
         cudaFreeHost(x->aux);
     if (x->pool)
@@ -670,50 +703,40 @@ aqua_set_state(aqua_ctx* x, uint32_t N, const aqua_vars* v, int on_host,
     cudaStream_t s = (cudaStream_t)stream;
     const size_t VS = (x->dims == 3) ? 4 : 2;
     VarSet& d = x->set[x->cur];
-    AQ_TRY(copy_in(d.id, v->id, N * 4ull, on_host, s));
-    AQ_TRY(copy_in(d.iset, v->iset, N * 4ull, on_host, s));
-    AQ_TRY(copy_in(d.imove, v->imove, N * 4ull, on_host, s));
-    AQ_TRY(copy_in(d.r, v->r, N * VS * 4, on_host, s));
-    AQ_TRY(copy_in(d.normal, v->normal, N * VS * 4, on_host, s));
-    AQ_TRY(copy_in(d.tangent, v->tangent, N * VS * 4, on_host, s));
-    if (v->binormal)
-        AQ_TRY(copy_in(d.binormal, v->binormal, N * VS * 4, on_host, s));
-    AQ_TRY(copy_in(d.u, v->u, N * VS * 4, on_host, s));
-    AQ_TRY(copy_in(d.dudt, v->dudt, N * VS * 4, on_host, s));
-    AQ_TRY(copy_in(d.rho, v->rho, N * 4ull, on_host, s));
-    AQ_TRY(copy_in(d.drhodt, v->drhodt, N * 4ull, on_host, s));
-    AQ_TRY(copy_in(d.m, v->m, N * 4ull, on_host, s));
-    AQ_TRY(copy_in(d.p, v->p, N * 4ull, on_host, s));
+    const void* required[] = { v->id, v->iset, v->imove, v->r, v->normal,
+                               v->tangent, v->u, v->dudt, v->rho, v->drhodt,
+                               v->m, v->p };
+    for (const void* p : required)
+        if (!p)
+            return AQUA_ERR_INVALID;
+    const Field f[] = { { d.id, v->id, N * 4ull }, { d.iset, v->iset, N * 4ull },
+                        { d.imove, v->imove, N * 4ull }, { d.r, v->r, N * VS * 4 },
+                        { d.normal, v->normal, N * VS * 4 },
+                        { d.tangent, v->tangent, N * VS * 4 },
+                        { d.binormal, v->binormal, N * VS * 4 },
+                        { d.u, v->u, N * VS * 4 }, { d.dudt, v->dudt, N * VS * 4 },
+                        { d.rho, v->rho, N * 4ull }, { d.drhodt, v->drhodt, N * 4ull },
+                        { d.m, v->m, N * 4ull }, { d.p, v->p, N * 4ull } };
     x->N = N;
     // the step scalars and one case holding every particle (aqua_set_cases()
-    // splits them), through the pinned staging area: asynchronous
-    uint8_t* st = stage_begin(x, kStageState);
-    if (!st)
-        return AQUA_ERR_CUDA;
-    DevScalars* hs = reinterpret_cast<DevScalars*>(st);
-    CaseScalars* c0 = reinterpret_cast<CaseScalars*>(st + kStageCs);
-    CaseMotion* m0 = reinterpret_cast<CaseMotion*>(st + kStageCm);
-    uint32_t* off = reinterpret_cast<uint32_t*>(st + kStageOff);
-    std::memset(hs, 0, sizeof(*hs));
-    std::memset(c0, 0, sizeof(*c0));
-    c0->t = t;
-    c0->dt = dt;
-    c0->iter = iter;
-    c0->dt_next = 0x7f800000u;
-    c0->cos_psi = c0->cos_psi_in = 1.f;
-    std::memset(m0, 0, sizeof(*m0));
-    off[0] = 0u;
-    off[1] = N;
+    // splits them): kernel arguments, so nothing is staged
+    StateRecords rec;
+    std::memset(&rec, 0, sizeof(rec));
+    rec.sc = x->sc;
+    rec.cs = x->cs;
+    rec.cm = x->cm;
+    rec.offsets = x->offsets;
+    rec.cid = d.cid;
+    rec.N = N;
+    rec.cs0.t = t;
+    rec.cs0.dt = dt;
+    rec.cs0.iter = iter;
+    rec.cs0.dt_next = 0x7f800000u;
+    rec.cs0.cos_psi = rec.cs0.cos_psi_in = 1.f;
     x->n_cases = 1;
     x->has_motion = 0;
-    AQ_CUDA(cudaMemcpyAsync(x->sc, hs, sizeof(*hs), cudaMemcpyHostToDevice, s));
-    AQ_CUDA(cudaMemcpyAsync(x->cs, c0, sizeof(*c0), cudaMemcpyHostToDevice, s));
-    AQ_CUDA(cudaMemcpyAsync(x->cm, m0, sizeof(*m0), cudaMemcpyHostToDevice, s));
-    AQ_CUDA(cudaMemcpyAsync(x->offsets, off, 2 * sizeof(uint32_t),
-                            cudaMemcpyHostToDevice, s));
-    AQ_CUDA(stage_done(x, kStageState, s));
-    AQ_CUDA(launch_set_case_ids(x->set[x->cur].cid, x->offsets, 1, N, s));
-    return AQUA_OK;
+    return copy_fields(x, f, sizeof(f) / sizeof(f[0]), on_host ? kHostToDevice : kOnDevice,
+                       rec, s);
 }
 
 aqua_status
@@ -724,21 +747,19 @@ aqua_get_state(aqua_ctx* x, aqua_vars* v, int on_host, void* stream)
     cudaStream_t s = (cudaStream_t)stream;
     const size_t N = x->N, VS = (x->dims == 3) ? 4 : 2;
     const VarSet& d = x->set[x->cur];
-    AQ_TRY(copy_out(v->id, d.id, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->iset, d.iset, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->imove, d.imove, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->r, d.r, N * VS * 4, on_host, s));
-    AQ_TRY(copy_out(v->normal, d.normal, N * VS * 4, on_host, s));
-    AQ_TRY(copy_out(v->tangent, d.tangent, N * VS * 4, on_host, s));
-    AQ_TRY(copy_out(v->binormal, d.binormal, N * VS * 4, on_host, s));
-    AQ_TRY(copy_out(v->u, d.u, N * VS * 4, on_host, s));
-    AQ_TRY(copy_out(v->dudt, d.dudt, N * VS * 4, on_host, s));
-    AQ_TRY(copy_out(v->rho, d.rho, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->drhodt, d.drhodt, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->m, d.m, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->p, d.p, N * 4, on_host, s));
-    AQ_TRY(copy_out(v->shepard, x->b.shepard, N * 4, on_host, s));
-    return AQUA_OK;
+    const Field f[] = { { v->id, d.id, N * 4 }, { v->iset, d.iset, N * 4 },
+                        { v->imove, d.imove, N * 4 }, { v->r, d.r, N * VS * 4 },
+                        { v->normal, d.normal, N * VS * 4 },
+                        { v->tangent, d.tangent, N * VS * 4 },
+                        { v->binormal, d.binormal, N * VS * 4 },
+                        { v->u, d.u, N * VS * 4 }, { v->dudt, d.dudt, N * VS * 4 },
+                        { v->rho, d.rho, N * 4 }, { v->drhodt, d.drhodt, N * 4 },
+                        { v->m, d.m, N * 4 }, { v->p, d.p, N * 4 },
+                        { v->shepard, x->b.shepard, N * 4 } };
+    StateRecords none;
+    std::memset(&none, 0, sizeof(none));
+    return copy_fields(x, f, sizeof(f) / sizeof(f[0]), on_host ? kDeviceToHost : kOnDevice,
+                       none, s);
 }
 
 aqua_status
@@ -880,7 +901,7 @@ aqua_set_cases(aqua_ctx* x, uint32_t n_cases, const uint32_t* offsets,
     cudaStream_t s = (cudaStream_t)stream;
     // the per-case records are built in the pinned staging area and copied
     // asynchronously
-    uint8_t* st = stage_begin(x, kStageCases);
+    uint8_t* st = stage_begin(x);
     if (!st)
         return AQUA_ERR_CUDA;
     CaseScalars* hs = reinterpret_cast<CaseScalars*>(st + kStageCs);
@@ -922,7 +943,7 @@ aqua_set_cases(aqua_ctx* x, uint32_t n_cases, const uint32_t* offsets,
         e = cudaMemcpyAsync(x->offsets, ho, (n_cases + 1) * sizeof(uint32_t),
                             cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = stage_done(x, kStageCases, s);
+        e = stage_done(x, s);
     if (e == cudaSuccess)
         e = launch_set_case_ids(x->set[x->cur].cid, x->offsets, n_cases, x->N, s);
     if (e != cudaSuccess) {

@@ -156,6 +156,31 @@ cudaError_t launch_finalize(DevScalars* sc, CaseScalars* cs,
                             cudaStream_t s);
 template<int D>
 cudaError_t launch_motion(const StepArgs& a, cudaStream_t s);
+// Copies between device arrays, all in one launch: `n` spans of `words` 32-bit
+// words; with `cid`, cid[0 .. N) = 0 and the records of a state of one case
+// are written as well (aqua_set_state).
+constexpr int kMaxSpans = 14;
+struct CopySpans
+{
+    uint32_t* dst[kMaxSpans];
+    const uint32_t* src[kMaxSpans];
+    uint64_t words[kMaxSpans];
+    int n;
+};
+struct StateRecords
+{
+    DevScalars* sc;
+    CaseScalars* cs;
+    CaseMotion* cm;
+    uint32_t* offsets;
+    uint32_t* cid;
+    uint32_t N;
+    DevScalars sc0;
+    CaseScalars cs0;
+    CaseMotion cm0;
+};
+cudaError_t launch_copy_spans(const CopySpans& spans, const StateRecords& rec,
+                              cudaStream_t s);
 cudaError_t launch_set_case_ids(uint32_t* cid, const uint32_t* offsets,
                                 uint32_t n_cases, uint32_t N, cudaStream_t s);
 cudaError_t launch_export_ihoc(const uint2* cells, uint32_t* ihoc,

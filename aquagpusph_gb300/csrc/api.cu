@@ -326,28 +326,39 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
     const uint32_t N = x->N;
     if (x->profiling)
         AQ_CUDA(cudaEventRecordWithFlags(x->ev[0], s, cudaEventRecordExternal));
-    AQ_CUDA(launch_begin(x->sc, x->cs, x->n_cases, b.cells, b.wall_range,
-                         x->consts.sample_on ? b.cell_mark : nullptr, x->ncap,
-                         N, b.sort_scratch, s));
+    uint8_t* mark = x->consts.sample_on ? b.cell_mark : nullptr;
     // one case: every particle's case id is 0 (not read)
     const uint32_t* cid = x->n_cases > 1 ? S.cid : nullptr;
-    if (x->dims == 3) {
-        AQ_CUDA(launch_minmax<3>(x->consts, S.r, S.imove, cid, N, x->cs,
-                                 x->sc, s));
-        AQ_CUDA(launch_ncells<3>(x->consts, x->cs, x->n_cases, x->sc, x->ncap, s));
-        AQ_CUDA(launch_icell_hist<3>(x->consts, S.r, S.imove, cid, N, x->cs,
-                                     x->sc, b.keys[0], b.sort_scratch,
-                                     x->passes, s));
+    if (N <= kSmallMax && x->n_cases <= kSmallCases) {
+        if (x->dims == 3)
+            AQ_CUDA(launch_small_linklist<3>(x->consts, S.r, S.imove, cid, N,
+                                             x->n_cases, x->cs, x->sc, b, mark,
+                                             x->ncap, x->passes, s));
+        else
+            AQ_CUDA(launch_small_linklist<2>(x->consts, S.r, S.imove, cid, N,
+                                             x->n_cases, x->cs, x->sc, b, mark,
+                                             x->ncap, x->passes, s));
     } else {
-        AQ_CUDA(launch_minmax<2>(x->consts, S.r, S.imove, cid, N, x->cs,
-                                 x->sc, s));
-        AQ_CUDA(launch_ncells<2>(x->consts, x->cs, x->n_cases, x->sc, x->ncap, s));
-        AQ_CUDA(launch_icell_hist<2>(x->consts, S.r, S.imove, cid, N, x->cs,
-                                     x->sc, b.keys[0], b.sort_scratch,
-                                     x->passes, s));
+        AQ_CUDA(launch_begin(x->sc, x->cs, x->n_cases, b.cells, b.wall_range,
+                             mark, x->ncap, N, b.sort_scratch, s));
+        if (x->dims == 3) {
+            AQ_CUDA(launch_minmax<3>(x->consts, S.r, S.imove, cid, N, x->cs,
+                                     x->sc, s));
+            AQ_CUDA(launch_ncells<3>(x->consts, x->cs, x->n_cases, x->sc, x->ncap, s));
+            AQ_CUDA(launch_icell_hist<3>(x->consts, S.r, S.imove, cid, N, x->cs,
+                                         x->sc, b.keys[0], b.sort_scratch,
+                                         x->passes, s));
+        } else {
+            AQ_CUDA(launch_minmax<2>(x->consts, S.r, S.imove, cid, N, x->cs,
+                                     x->sc, s));
+            AQ_CUDA(launch_ncells<2>(x->consts, x->cs, x->n_cases, x->sc, x->ncap, s));
+            AQ_CUDA(launch_icell_hist<2>(x->consts, S.r, S.imove, cid, N, x->cs,
+                                         x->sc, b.keys[0], b.sort_scratch,
+                                         x->passes, s));
+        }
+        AQ_CUDA(launch_radix_passes(b.keys, b.vals, N, x->passes, b.sort_scratch,
+                                    true, x->sc, s));
     }
-    AQ_CUDA(launch_radix_passes(b.keys, b.vals, N, x->passes, b.sort_scratch,
-                                true, x->sc, s));
     StepArgs a;
     a.N = N;
     a.ncap = x->ncap;
@@ -586,7 +597,9 @@ aqua_create(const aqua_params* params, uint32_t capacity,
     // blocks of 8 warps per SM; elsewhere the direct sweep with prefetch at
     // 28 warps per SM (see enqueue_step)
     x->sweep_grid = (unsigned)x->sms * kSweepClusteredBlocks;
-    if (fast::prepare_sweep_cl() != cudaSuccess) {
+    if (fast::prepare_sweep_cl() != cudaSuccess ||
+        (x->dims == 3 ? prepare_small_linklist<3>() : prepare_small_linklist<2>()) !=
+            cudaSuccess) {
         delete x;
         return AQUA_ERR_CUDA;
     }

@@ -93,6 +93,22 @@ cudaError_t launch_begin(DevScalars* sc, CaseScalars* cs, uint32_t n_cases,
                          uint2* cells, uint2* wall_range, uint8_t* cell_mark,
                          uint32_t ncap, uint32_t N, uint32_t* sort_scratch,
                          cudaStream_t s);
+// all of it in one launch, for at most kSmallMax particles and kSmallCases
+// cases: keys and permutation in keys / vals[passes & 1].  Whole steps with
+// it and with the separate kernels: 42 against 55 us for 8,206 particles, 147
+// against 161 for 15,640 and 98 against 104 for 46,600 in 5 cases; at 57,600
+// they are equal (558 and 555), so the line lies between.
+constexpr uint32_t kSmallMax = 49152;
+constexpr uint32_t kSmallCases = 32;   // one lane each
+template<int D>
+cudaError_t prepare_small_linklist();
+template<int D>
+cudaError_t launch_small_linklist(const Consts& c, const float* r,
+                                  const int32_t* imove, const uint32_t* cid,
+                                  uint32_t N, uint32_t n_cases, CaseScalars* cs,
+                                  DevScalars* sc, const StepBufs& b,
+                                  uint8_t* cell_mark, uint32_t ncap,
+                                  uint32_t passes, cudaStream_t s);
 template<int D>
 cudaError_t launch_minmax(const Consts& c, const float* r, const int32_t* imove,
                           const uint32_t* cid, uint32_t N, CaseScalars* cs,

@@ -20,6 +20,10 @@
 #include "aqua_internal.cuh"
 #include "kernels.cuh"
 
+#include <cooperative_groups.h>
+
+namespace cg = cooperative_groups;
+
 namespace aqua {
 
 namespace {
@@ -27,7 +31,7 @@ namespace {
 __device__ __forceinline__ void
 atomic_min_float(float* addr, float v)
 {
-    if (v >= 0.f)
+    if (__float_as_int(v) >= 0)
         atomicMin((int*)addr, __float_as_int(v));
     else
         atomicMax((unsigned int*)addr, __float_as_uint(v));
@@ -36,7 +40,7 @@ atomic_min_float(float* addr, float v)
 __device__ __forceinline__ void
 atomic_max_float(float* addr, float v)
 {
-    if (v >= 0.f)
+    if (__float_as_int(v) >= 0)
         atomicMax((int*)addr, __float_as_int(v));
     else
         atomicMin((unsigned int*)addr, __float_as_uint(v));
@@ -324,8 +328,9 @@ cell_of(const Consts& c, const float x[4], const float r_min[4],
         const uint32_t n[4])
 {
     uint32_t a[3] = { 0u, 0u, 0u };
+    // x lies in the box and the box's cells were counted below 2^32
     for (int k = 0; k < D; k++)
-        a[k] = (uint32_t)(unsigned long long)((x[k] - r_min[k]) * c.idist) + 2u;
+        a[k] = (uint32_t)((x[k] - r_min[k]) * c.idist) + 2u;
     uint32_t cell = a[0] + a[1] * n[0];
     if (D == 3)
         cell += a[2] * n[0] * n[1];
@@ -632,6 +637,332 @@ k_onesweep(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
     }
 }
 
+// The whole link-list of a small step (at most kSmallMax particles and
+// kSmallCases cases) in one launch: a cluster of 8 blocks keeps keys and
+// 16-bit indices in its shared memory, reduces the boxes, computes n_cells and
+// the keys and sorts them, each pass written straight into the next holder's
+// shared memory; the other clusters clear the cell table meanwhile.  The
+// separate kernels (k_begin, k_minmax, k_ncells, k_icell_hist and two or three
+// k_onesweep) are 4 to 9 us each at this size, all of it launch and latency:
+// 38 us in all for 8,206 particles, here 13 (46,600: 39, here 21).  What is
+// left is latency too: a cluster barrier is 0.5 us, two a pass.
+constexpr int kSmallThreads = 1024;
+constexpr uint32_t kSmallBlocks = 8;
+constexpr uint32_t kSmallPer = kSmallMax / kSmallBlocks;  // keys per block
+constexpr uint32_t kSmallItems = kSmallPer / kSmallThreads;
+struct SmallSmem
+{
+    uint32_t key[2][kSmallPer];
+    uint16_t val[2][kSmallPer];
+    uint16_t hist[kSmallThreads / 32][256];  // per warp, then first places
+    uint32_t count[256];                     // the block's keys of each digit
+    uint32_t digit[256];                     // first place of each digit
+    float box[kSmallCases][8];               // this block's r_min, r_max
+    float r_min[kSmallCases][4];
+    uint32_t n[kSmallCases][4];              // n_cells, first cell
+    uint32_t warp[8];
+    uint32_t bad, stop, cells;
+};
+
+template<int D>
+__global__ void __launch_bounds__(kSmallThreads)
+k_small_linklist(Consts c, const float* r, const int32_t* imove,
+                 const uint32_t* cid, uint32_t N, uint32_t n_cases,
+                 CaseScalars* cs, DevScalars* sc, uint2* cells,
+                 uint2* wall_range, uint8_t* cell_mark, uint32_t ncap,
+                 uint32_t* keys_out, uint32_t* vals_out)
+{
+    constexpr int VS = Vec<D>::VS;
+    constexpr int NW = kSmallThreads / 32;
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (blockIdx.x >= kSmallBlocks) {
+        if (__syncthreads_or(t == 0 && sc->err))
+            return;
+        const uint32_t stride = (gridDim.x - kSmallBlocks) * kSmallThreads;
+        for (uint32_t k = (blockIdx.x - kSmallBlocks) * kSmallThreads + t;
+             k < ncap; k += stride) {
+            cells[k] = make_uint2(N, N);
+            wall_range[k] = make_uint2(0xffffffffu, 0u);
+            if (cell_mark)
+                cell_mark[k] = 0;
+        }
+        return;
+    }
+    const cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t b = blockIdx.x;  // = the rank in the first cluster
+    extern __shared__ __align__(16) uint8_t small_raw[];
+    SmallSmem& S = *reinterpret_cast<SmallSmem*>(small_raw);
+    if (b == 0 && t == 0) {
+        sc->n_chunks = 0;
+        sc->chunk_next = 0;
+    }
+    // an error of an earlier step: the blocks read it before any of this
+    // launch's blocks can set it (rank 0, after the second cluster barrier)
+    if (t == 0) {
+        S.stop = sc->err;
+        S.bad = 0;
+    }
+    if (t < n_cases) {
+        for (int d = 0; d < 4; d++) {
+            S.box[t][d] = INFINITY;
+            S.box[t][4 + d] = -INFINITY;
+        }
+        if (b == 0)
+            cs[t].dt_next = __float_as_uint(INFINITY);
+    }
+    __syncthreads();
+    const uint32_t stop = S.stop;
+    // block b holds positions [b * per, b * per + cnt), warp w of it those
+    // from w * seg
+    const uint32_t per = ((N + kSmallBlocks - 1) / kSmallBlocks + 31u) & ~31u;
+    const uint32_t first = b * per;
+    const uint32_t cnt = first < N ? min(per, N - first) : 0u;
+    const uint32_t seg = (per + kSmallThreads - 1) / kSmallThreads * 32u;
+    float xs[kSmallItems][VS];
+    if (!stop) {
+        // boxes (min and max are exact in any order); every load is issued
+        // before the first is used
+        uint32_t ks[kSmallItems];
+#pragma unroll
+        for (uint32_t it = 0; it < kSmallItems; it++) {
+            const uint32_t i = warp * seg + it * 32 + lane;
+            float x[4] = { 0.f, 0.f, 0.f, 0.f };
+            ks[it] = 0;
+            if (it * 32 < seg && i < cnt) {
+                bool removed;
+                domain_position<D>(c, r, imove, first + i, x, removed);
+                ks[it] = cid ? cid[first + i] : 0u;
+            }
+            for (int d = 0; d < VS; d++)
+                xs[it][d] = x[d];
+        }
+        const uint32_t k0 = __shfl_sync(0xffffffffu, ks[0], 0);
+        bool bad = false, same = true;
+        float mn[VS], mx[VS];
+        for (int d = 0; d < VS; d++) {
+            mn[d] = INFINITY;
+            mx[d] = -INFINITY;
+        }
+#pragma unroll
+        for (uint32_t it = 0; it < kSmallItems; it++) {
+            const uint32_t i = warp * seg + it * 32 + lane;
+            if (it * 32 < seg && i < cnt) {
+                same = same && ks[it] == k0;
+                for (int d = 0; d < VS; d++) {
+                    const bool ok = isfinite(xs[it][d]);
+                    bad = bad || !ok;
+                    mn[d] = cl_min(mn[d], ok ? xs[it][d] : INFINITY);
+                    mx[d] = cl_max(mx[d], ok ? xs[it][d] : -INFINITY);
+                }
+            }
+        }
+        if (__all_sync(0xffffffffu, same)) {
+            for (int d = 0; d < VS; d++) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    mn[d] = cl_min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
+                    mx[d] = cl_max(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+                }
+                if (lane == 0) {
+                    atomic_min_float(&S.box[k0][d], mn[d]);
+                    atomic_max_float(&S.box[k0][4 + d], mx[d]);
+                }
+            }
+        } else {  // the few warps at a case's end
+#pragma unroll
+            for (uint32_t it = 0; it < kSmallItems; it++) {
+                const uint32_t i = warp * seg + it * 32 + lane;
+                if (it * 32 < seg && i < cnt)
+                    for (int d = 0; d < VS; d++)
+                        if (isfinite(xs[it][d])) {
+                            atomic_min_float(&S.box[ks[it]][d], xs[it][d]);
+                            atomic_max_float(&S.box[ks[it]][4 + d], xs[it][d]);
+                        }
+            }
+        }
+        if (bad)
+            S.bad = 1;
+    }
+    cluster.sync();
+    // n_cells and the first cells as k_ncells, every block for itself: lane
+    // k = case k
+    if (!stop && warp == 0) {
+        float box[8];
+        for (int d = 0; d < 4; d++) {
+            box[d] = INFINITY;
+            box[4 + d] = -INFINITY;
+        }
+        uint32_t bad = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kSmallBlocks; q++) {
+            const SmallSmem& Q = *cluster.map_shared_rank(&S, q);
+            bad |= Q.bad;
+            if (lane < n_cases)
+                for (int d = 0; d < VS; d++) {
+                    box[d] = cl_min(box[d], Q.box[lane][d]);
+                    box[4 + d] = cl_max(box[4 + d], Q.box[lane][4 + d]);
+                }
+        }
+        unsigned long long n[3] = { 1, 1, 1 };
+        bool over = false;
+        if (lane < n_cases)
+            for (int d = 0; d < D; d++) {
+                const float span = (box[4 + d] - box[d]) / c.cell_length;
+                if (!(span >= 0.f) || span > 4.0e9f)
+                    over = true;
+                else
+                    n[d] = (unsigned long long)span + 6ull;
+            }
+        const unsigned long long mine =
+            lane < n_cases ? n[0] * n[1] * n[2] : 0ull;
+        unsigned long long sum = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= (uint32_t)o)
+                sum += y;
+        }
+        const unsigned long long total = __shfl_sync(0xffffffffu, sum, 31);
+        over = __any_sync(0xffffffffu, over) || total > ncap;
+        const uint32_t base = (uint32_t)(sum - mine);
+        if (lane < n_cases) {
+            for (int d = 0; d < 4; d++)
+                S.r_min[lane][d] = box[d];
+            for (int d = 0; d < 3; d++)
+                S.n[lane][d] = (uint32_t)n[d];
+            S.n[lane][3] = base;
+            if (b == 0) {
+                CaseScalars& k = cs[lane];
+                for (int d = 0; d < 4; d++) {
+                    k.r_min[d] = box[d];
+                    k.r_max[d] = box[4 + d];
+                }
+                if (!bad && !over) {
+                    for (int d = 0; d < 3; d++)
+                        k.n_cells[d] = (uint32_t)n[d];
+                    k.n_cells[3] = (uint32_t)mine;
+                    k.cell_base = base;
+                }
+            }
+        }
+        if (lane == 0) {
+            S.stop = bad || over;
+            S.cells = (uint32_t)total;
+            if (b == 0 && !bad && !over)
+                sc->total_cells = (uint32_t)total;
+            if (b == 0 && (bad || over))
+                atomicOr(&sc->err, bad ? kErrNonFinite : kErrCapacity);
+        }
+    }
+    __syncthreads();
+    if (S.stop) {  // the same in every block
+        cluster.sync();  // every block has read the boxes and flags
+        return;
+    }
+#pragma unroll
+    for (uint32_t it = 0; it < kSmallItems; it++) {
+        const uint32_t i = warp * seg + it * 32 + lane;
+        if (it * 32 < seg && i < cnt) {
+            const uint32_t k = cid ? cid[first + i] : 0u;
+            S.key[0][i] = S.n[k][3] + cell_of<D>(c, xs[it], S.r_min[k], S.n[k]);
+            S.val[0][i] = (uint16_t)(first + i);
+        }
+    }
+    // at / per for at < 2^16 and per <= 2^13: the product's excess over the
+    // quotient is below 2^-16, less than 1 / per
+    const uint32_t over_per = 0xffffffffu / per + 1u;
+    const unsigned lt = (1u << lane) - 1u;
+    // the digits that the cells of this step have
+    const uint32_t passes = max(39u - (uint32_t)__clz(S.cells - 1u), 8u) / 8u;
+    for (uint32_t p = 0; p < passes; p++) {
+        const uint32_t* ki = S.key[p & 1];
+        const uint16_t* vi = S.val[p & 1];
+        for (uint32_t k = t; k < NW * 128u; k += kSmallThreads)
+            reinterpret_cast<uint32_t*>(S.hist)[k] = 0;
+        __syncthreads();
+        // stable ranks within the warp's positions
+        uint32_t rank[kSmallItems];
+#pragma unroll
+        for (uint32_t it = 0; it < kSmallItems; it++) {
+            if (it * 32 >= seg)
+                break;
+            const uint32_t i = warp * seg + it * 32 + lane;
+            const bool valid = i < cnt;
+            const uint32_t d = valid ? (ki[i] >> (8 * p)) & 255u : 256u;
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            const uint32_t before = valid ? S.hist[warp][d] : 0u;
+            __syncwarp();
+            if (valid && lane == (uint32_t)__ffs(peers) - 1u)
+                S.hist[warp][d] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+            rank[it] = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        // thread t = digit t: the warps' offsets and the block's count
+        if (t < 256) {
+            uint32_t v[NW], sum = 0;
+#pragma unroll
+            for (int w = 0; w < NW; w++)
+                v[w] = S.hist[w][t];
+#pragma unroll
+            for (int w = 0; w < NW; w++) {
+                S.hist[w][t] = (uint16_t)sum;
+                sum += v[w];
+            }
+            S.count[t] = sum;
+        }
+        cluster.sync();
+        // the digits' first places, and the blocks before this one
+        uint32_t all = 0, before = 0;
+        if (t < 256)
+#pragma unroll
+            for (uint32_t q = 0; q < kSmallBlocks; q++) {
+                const uint32_t v = cluster.map_shared_rank(&S, q)->count[t];
+                all += v;
+                before += q < b ? v : 0u;
+            }
+        const bool last = p + 1 == passes;
+        if (last)  // no shared memory of another block is used from here on
+            cluster.barrier_arrive();
+        uint32_t x = all;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= (uint32_t)o)
+                x += y;
+        }
+        if (t < 256 && lane == 31)
+            S.warp[warp] = x;
+        __syncthreads();
+        if (t < 256) {
+            uint32_t w0 = 0;
+            for (uint32_t w = 0; w < warp; w++)
+                w0 += S.warp[w];
+            S.digit[t] = w0 + x - all + before;
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t it = 0; it < kSmallItems; it++) {
+            const uint32_t i = warp * seg + it * 32 + lane;
+            if (it * 32 < seg && i < cnt) {
+                const uint32_t key = ki[i], d = (key >> (8 * p)) & 255u;
+                const uint32_t at = S.digit[d] + S.hist[warp][d] + rank[it];
+                if (last) {
+                    keys_out[at] = key;
+                    vals_out[at] = vi[i];
+                } else {
+                    const uint32_t q = __umulhi(at, over_per);
+                    SmallSmem& Q = *cluster.map_shared_rank(&S, q);
+                    Q.key[(p + 1) & 1][at - q * per] = key;
+                    Q.val[(p + 1) & 1][at - q * per] = vi[i];
+                }
+            }
+        }
+        // every key has arrived; the counts have been read
+        if (last)
+            cluster.barrier_wait();
+        else
+            cluster.sync();
+    }
+}
+
 // inverse permutation (optional output of the sort tool)
 __global__ void
 k_inverse_perm(const uint32_t* perm, uint32_t* inv, uint32_t n,
@@ -804,6 +1135,44 @@ launch_icell_hist(const Consts& c, const float* r, const int32_t* imove,
     return cudaGetLastError();
 }
 
+template<int D>
+cudaError_t
+prepare_small_linklist()
+{
+    return cudaFuncSetAttribute(k_small_linklist<D>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(SmallSmem));
+}
+
+template<int D>
+cudaError_t
+launch_small_linklist(const Consts& c, const float* r, const int32_t* imove,
+                      const uint32_t* cid, uint32_t N, uint32_t n_cases,
+                      CaseScalars* cs, DevScalars* sc, const StepBufs& b,
+                      uint8_t* cell_mark, uint32_t ncap, uint32_t passes,
+                      cudaStream_t s)
+{
+    const unsigned clear = min(
+        max((ncap + kSmallBlocks * kSmallThreads - 1) / (kSmallBlocks * kSmallThreads), 1u),
+        16u);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kSmallBlocks;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSmallBlocks * (1 + clear));
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = sizeof(SmallSmem);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_small_linklist<D>, c, r, imove, cid, N,
+                              n_cases, cs, sc, b.cells, b.wall_range, cell_mark,
+                              ncap, b.keys[passes & 1],
+                              b.vals[passes & 1]);
+}
+
 cudaError_t
 launch_inverse_perm(const uint32_t* perm, uint32_t* inv, uint32_t n,
                     const DevScalars* sc, cudaStream_t s)
@@ -833,6 +1202,16 @@ launch_iota(uint32_t* p, uint32_t n, cudaStream_t s)
     return cudaGetLastError();
 }
 
+template cudaError_t prepare_small_linklist<2>();
+template cudaError_t prepare_small_linklist<3>();
+template cudaError_t launch_small_linklist<2>(
+    const Consts&, const float*, const int32_t*, const uint32_t*, uint32_t,
+    uint32_t, CaseScalars*, DevScalars*, const StepBufs&, uint8_t*, uint32_t,
+    uint32_t, cudaStream_t);
+template cudaError_t launch_small_linklist<3>(
+    const Consts&, const float*, const int32_t*, const uint32_t*, uint32_t,
+    uint32_t, CaseScalars*, DevScalars*, const StepBufs&, uint8_t*, uint32_t,
+    uint32_t, cudaStream_t);
 template cudaError_t launch_minmax<2>(const Consts&, const float*,
                                       const int32_t*, const uint32_t*, uint32_t,
                                       CaseScalars*, DevScalars*, cudaStream_t);

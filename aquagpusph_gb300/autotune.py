@@ -31,10 +31,13 @@ VARIANTS = ((0, 128, 128, 24), (1, 64, 128, 24), (2, 64, 64, 24),
 # resident warps per SM tried for each variant (blocks = warps * 32 / threads)
 WARPS_PER_SM = (8, 12, 16, 20, 24, 28, 32, 36)
 MAX_BLOCKS_PER_SM = 32
-# the clustered sweep of the fast 3-D build (BIe walls, midpoint scheme):
-# (variant, threads per block, blocks per SM tried); 15 and 17 hold at most
-# 2 blocks per SM, 16 at most 3 (shared memory, registers)
-CLUSTERED = ((15, 256, (1, 2)), (16, 256, (1, 2, 3)), (17, 384, (1, 2)))
+# the default variant: the clustered sweep of the fast 3-D build (BIe walls,
+# midpoint scheme; 256 threads, 1 to 3 blocks per SM tried), and everywhere
+# else the quad sweep (128 threads; its grid is fixed).  The quad sweep is 1.2
+# to 3.4 times as fast as the variants above, which are kept for their own
+# error cases and saved choices
+CLUSTERED = (16, 256, (1, 2, 3))
+QUAD = (16, 128, (3,))
 
 
 def cache_path() -> str:
@@ -55,6 +58,7 @@ def gpu_name() -> str:
 
 
 def signature(solver, fast: bool) -> str:
+    # "quad": choices saved when there was no quad sweep do not apply
     p = solver.params
     n_cases = getattr(solver, "n_cases", 1)
     # particle counts bucketed to 1/16 of a power of two
@@ -62,7 +66,7 @@ def signature(solver, fast: bool) -> str:
     bucket = 1 << (n.bit_length() - 1)
     bucket = bucket + ((n - bucket) // (bucket // 16 or 1)) * (bucket // 16 or 1)
     return (f"{gpu_name()}|dims={p.dims}|N~{bucket}|cases={n_cases}|"
-            f"h={p.h:.6g}|{'fast' if fast else 'exact'}")
+            f"h={p.h:.6g}|{'fast' if fast else 'exact'}|quad")
 
 
 def _load():
@@ -101,10 +105,9 @@ def candidates(clustered: bool = False):
             b = w * 32 // threads
             if b * threads == w * 32 and 1 <= b <= MAX_BLOCKS_PER_SM:
                 yield v, b
-    if clustered:
-        for v, threads, blocks in CLUSTERED:
-            for b in blocks:
-                yield v, b
+    v, _, blocks = CLUSTERED if clustered else QUAD
+    for b in blocks:
+        yield v, b
 
 
 def autotune(solver, fast: bool, steps: int = 3, use_cache: bool = True,
@@ -119,7 +122,8 @@ def autotune(solver, fast: bool, steps: int = 3, use_cache: bool = True,
         solver.set_tuning(v, b)
         return dict(cache[key], cached=True)
     results = []
-    for v, b in candidates(clustered_applies(solver, fast)):
+    clustered = clustered_applies(solver, fast)
+    for v, b in candidates(clustered):
         try:
             solver.set_tuning(v, b)
         except _lib.AquaError:
@@ -135,7 +139,8 @@ def autotune(solver, fast: bool, steps: int = 3, use_cache: bool = True,
     results.sort()
     best_dt, v, b = results[0]
     solver.set_tuning(v, b)
-    threads = dict((x[0], x[1]) for x in VARIANTS + CLUSTERED)
+    threads = dict((x[0], x[1]) for x in
+                   VARIANTS + ((CLUSTERED if clustered else QUAD),))
     entry = {"variant": v, "blocks_per_sm": b,
              "threads": threads[v],
              "queue": dict((x[0], x[2]) for x in VARIANTS).get(v, 0),

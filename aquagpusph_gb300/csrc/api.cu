@@ -304,6 +304,12 @@ stage_done(aqua_ctx* x, cudaStream_t s)
     return cudaEventRecord(x->stage_ev[x->stage_cur], s);
 }
 
+bool
+small_linklist(const aqua_ctx* x)
+{
+    return x->N <= kSmallMax && x->n_cases <= kSmallCases;
+}
+
 // The clustered sweep runs for the fast build in 3-D with BIe walls and the
 // midpoint scheme when the chosen variant is a clustered one
 bool
@@ -329,7 +335,7 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
     uint8_t* mark = x->consts.sample_on ? b.cell_mark : nullptr;
     // one case: every particle's case id is 0 (not read)
     const uint32_t* cid = x->n_cases > 1 ? S.cid : nullptr;
-    if (N <= kSmallMax && x->n_cases <= kSmallCases) {
+    if (small_linklist(x)) {
         if (x->dims == 3)
             AQ_CUDA(launch_small_linklist<3>(x->consts, S.r, S.imove, cid, N,
                                              x->n_cases, x->cs, x->sc, b, mark,
@@ -594,8 +600,8 @@ aqua_create(const aqua_params* params, uint32_t capacity,
     }
     x->sms = sms > 0 ? sms : 1;
     // untuned default: the clustered sweep (fast 3-D BIe midpoint) with 3
-    // blocks of 8 warps per SM; elsewhere the direct sweep with prefetch at
-    // 28 warps per SM (see enqueue_step)
+    // blocks of 8 warps per SM; elsewhere the quad sweep, whose grid is its
+    // own (see enqueue_step)
     x->sweep_grid = (unsigned)x->sms * kSweepClusteredBlocks;
     if (fast::prepare_sweep_cl() != cudaSuccess ||
         (x->dims == 3 ? prepare_small_linklist<3>() : prepare_small_linklist<2>()) !=
@@ -1168,11 +1174,10 @@ aqua_launches_per_step(aqua_ctx* x)
 {
     if (!x)
         return 0;
-    // begin, minmax, ncells, icell+hist, (passes - 1) hist,
-    // passes x (scan, scatter), gather, [BI walls,] chunks or (cell list,
-    // clusters), sweep, finalize [, motion]
-    return 4u + (x->passes - 1u) + 2u * x->passes + 4u +
-           (sweep_clustered(x) ? 1u : 0u) +
+    // link-list (one launch, or begin, minmax, ncells, icell+hist and the
+    // radix passes), gather, clusters or chunks, [BI walls,] sweep, finalize
+    // [, motion]
+    return (small_linklist(x) ? 1u : 4u + x->passes) + 4u +
            (x->consts.boundary == AQUA_BOUNDARY_BI ? 1u : 0u) +
            (x->has_motion ? 1u : 0u);
 }

@@ -17,21 +17,13 @@ constexpr int kSortTile = kSortThreads * kSortItems;   // keys per block
 // prefetched by asynchronous copies: 7 = 64 threads, 8 = 128 threads;
 // those with the register budget of 28 resident warps per SM (9 = 64,
 // 10 = 128 threads), 32 (11, 12) or 36 (13, 14)
-// the clustered sweep of the fast 3-D build (BIe walls, midpoint scheme):
-// 15 = 8 warps per block for 2 blocks per SM, 16 = 8 warps for 3 blocks,
-// 17 = 12 warps for 2 blocks; each stages 2,048 neighbour records per pass
+// 15 to 17: the clustered sweep of the fast 3-D build (BIe walls, midpoint
+// scheme; 8 warps per block, 2,048 neighbour records staged per pass), the quad
+// sweep everywhere else
 constexpr int kSweepClustered = 15;
 constexpr int kSweepVariants = 18;
 constexpr int kSweepClusteredDefault = 16;
 constexpr unsigned kSweepClusteredBlocks = 3;
-inline int
-sweep_variant_threads(int v)
-{
-    if (v >= kSweepClustered)
-        return v == kSweepClustered + 2 ? 384 : 256;
-    return (v == 0 || (v >= 6 && v % 2 == 0)) ? 128 : 64;
-}
-
 // Wendland C2 (Wendland{2D,3D}.hcl:44-66): the constant factors of W and F;
 // float products folded at compile time, as the OpenCL compiler folds them
 template<int D>

@@ -363,10 +363,10 @@ k_motion(StepArgs a)
 }
 
 // One launch for the copies of a state (and its records): a copy call each
-// costs 2 us and more a field on the GPU, 27 fields a state in and out (5 tanks,
-// 46,545 particles: 296 us a pass, now 209; 406,402 in 3-D: 1,029, now 866).  Sixteen-byte words where
-// both ends are aligned to them; the rows of the grid's y dimension are the
-// spans.
+// costs 2 us and more a field on the GPU, 27 fields a state in and out (5
+// tanks, 46,545 particles: 296 us a pass, then 209; 406,402 in 3-D: 1,029,
+// then 866).  Sixteen-byte words where both ends are aligned to them; the rows
+// of the grid's y dimension are the spans.
 constexpr int kSpanThreads = 256;
 __global__ void __launch_bounds__(kSpanThreads)
 k_copy_spans(CopySpans sp, StateRecords rec)

@@ -510,9 +510,10 @@ def run_ours(args):
     sweep_b = SWEEP_BYTES_3D if three_d else SWEEP_BYTES_2D
     step_b = STEP_BYTES_3D if three_d else STEP_BYTES_2D
     achieved = sweep_b * c.N / (stage_ms["sweep"] * 1e-3) / 1e9
-    clustered = (three_d and args.precision == "fast" and
-                 (tuning is None or tuning["variant"] >= 15))
-    kname = ("k_sweep_cl" if clustered else "k_sweep") + ("<3>" if three_d else "<2>")
+    default = tuning is None or tuning["variant"] >= 15
+    clustered = three_d and args.precision == "fast" and default
+    kname = (("k_sweep_cl" if clustered else "k_sweep_quad" if default else "k_sweep") +
+             ("<3>" if three_d else "<2>"))
     traffic_pp = load_traffic(kname)
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved,
                 "peak": peak, "unit": "GB/s", "frac": achieved / peak,

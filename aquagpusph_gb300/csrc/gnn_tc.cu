@@ -324,24 +324,30 @@ k_linear_fwd_tc(uint32_t M, uint32_t K, const uint16_t* __restrict__ X,
 // ---------------------------------------------------------------------------
 // Fused three-layer edge MLP: Y = L3(act(L2(act(L1(X))))) on tiles of 128
 // edges, every activation kept on chip.  The layer-1 input of each tile is
-// gathered into shared memory (core-matrix layout) by asynchronous copies:
-// rows of X, or, in PAIR mode, the concatenation [H[recv[e]] (64),
+// gathered into shared memory by asynchronous copies: rows of X, or, in PAIR mode, the concatenation [H[recv[e]] (64),
 // H[send[e]] (64), Ef[e] (16)] that aqua_gnn_gather_pair materialises.  The
-// three layers share one 64-column tensor-memory accumulator; each epilogue
-// reads it back (tcgen05.ld), adds the bias, applies the activation, rounds
+// layers accumulate in 64 columns of tensor memory (layer 1 in its own, layers 2
+// and 3 in turn); each epilogue reads them back (tcgen05.ld), adds the bias, applies the activation, rounds
 // to BF16 and writes the next layer's A operand into shared memory, exactly
 // the values the unfused layers store to and reload from global memory, so
 // the result is bit-identical to three aqua_gnn_linear_fwd_tc calls.  Only
 // the BF16 output of layer 3 is written.  A wait that times out sets *err;
-// the CTA finishes that tile (its outputs are then not to be trusted) and
+// the group finishes that tile (its outputs are then not to be trusted) and
 // stops.
 //
+// The tile's chain of layers, barriers and sums bounds it, not the tensor pipe
+// (10%) nor memory: three groups a CTA run three chains, and a warp of each
+// takes the gather and layer 1 of the next tile off the chain (eight warps that
+// gathered themselves stood 3,000 cycles of 18,000 in the copies' queue).  40.4M
+// edges: pair input 5.8 ms with three CTAs of 8 warps an SM, 5.1 with the
+// gathering warp, 3.9 with swizzled rows; 16-wide input 3.5 and 3.6.
+//
 // With SUM the layer-3 output never leaves the chip either: it is summed
-// into the receivers (aqua_gnn_segment_sum fused in).  Each CTA owns a
-// contiguous range of receivers (about E / grid edges) and walks its edges
+// into the receivers (aqua_gnn_segment_sum fused in).  Each group owns a
+// contiguous range of receivers (about E / groups edges) and walks its edges
 // in 128-edge tiles, in order.  The layer-3 tile is staged in shared memory
 // (row-major, 16-byte groups XOR-swizzled by row), the receivers' runs of
-// rows are summed by the warps (run k by warp k mod 4, lanes over column
+// rows are summed by the warps (run k by warp k mod 8, lanes over column
 // pairs), and a receiver whose edges continue in the next tile carries its
 // partial sums there.  Every receiver's sum is thus the same sequence of
 // FP32 additions, in edge order from zero, as aqua_gnn_segment_sum's: the
@@ -356,51 +362,60 @@ cp_async_16z(void* dst, const void* src, bool valid)
                  : "memory");
 }
 
-// bytes of the operand buffer: the layer-1 input or a 128 x 64 bf16 tile
+// bytes of the layer-1 operand buffer, and of the activation buffer (128 x 64)
 template<int K1>
 __host__ __device__ constexpr uint32_t
 edge_operand_bytes()
 {
-    constexpr uint32_t a0 = ((128u * K1 * 2u + 1023u) / 1024u) * 1024u;
-    constexpr uint32_t a1 = 128u * 64u * 2u;
-    return a0 > a1 ? a0 : a1;
+    return ((128u * K1 * 2u + 1023u) / 1024u) * 1024u;
 }
+constexpr uint32_t kEdgeAct = 128u * 64u * 2u;
 
-// 8 warps: warps w and w + 4 read the same 32 tensor-memory lanes (rows
-// 32 (w % 4) ..), each one half of the 64 columns
+// A CTA is kEdgeGroups groups that share the weights; each walks its own tiles
+// and has its own barriers, accumulators and buffers.  Eight warps of a group
+// read the accumulators (warps w and w + 4 the same 32 tensor-memory lanes, rows
+// 32 (w % 4) .., each one half of the 64 columns); a ninth gathers the layer-1
+// input of the next tile and issues its MMAs meanwhile.
 constexpr int kEdgeThreads = 256;
 constexpr int kEdgeWarps = kEdgeThreads / 32;
+constexpr int kEdgeGroups = 3;
+constexpr int kEdgeBlock = kEdgeGroups * (kEdgeThreads + 32);
+constexpr uint32_t kEdgeTmem = 512;  // columns: 128 a group, a power of two
 
-// shared memory after the two operand buffers: the biases, and the
-// receiver-sum bookkeeping of a SUM CTA
+// shared memory after a group's two buffers: the receiver-sum bookkeeping
 struct EdgeShared {
-    float bias[3][64];
     uint32_t recv[kTcRows];   // receiver of each row of the tile (~0: none)
     uint32_t start[4];        // rows that start a receiver's run, per 32 rows
     float carry[2][64];       // partial sums carried into the next tile
     uint32_t carry_node[2];   // their receiver (~0: none)
-    uint32_t nodes[2];        // this CTA's receivers [nodes[0], nodes[1])
+    uint32_t nodes[2];        // this group's receivers [nodes[0], nodes[1])
     uint32_t next_recv;       // receiver of the edge after the tile (~0: none)
+    uint32_t stop;            // the group gave up: no further tile is gathered
+    uint32_t pad[2];
 };
+static_assert(sizeof(EdgeShared) % 16 == 0, "buffers stay aligned");
 
-// CTAs per SM: three of 256 threads (registers); operand buffers per CTA:
-// one with the 144-wide pair input (shared memory), two with the 16-wide
-// rows (the next tile's rows are gathered during this tile's layers)
-template<bool PAIR>
-__host__ __device__ constexpr int
-edge_ctas_per_sm()
+// barrier of one group, with the or of `v` over its threads
+__device__ __forceinline__ void
+group_sync(uint32_t group)
 {
-    return 3;
+    asm volatile("barrier.sync %0, %1;\n" :: "r"(group + 1u), "r"((uint32_t)kEdgeThreads)
+                 : "memory");
 }
-template<bool PAIR>
-__host__ __device__ constexpr uint32_t
-edge_buffers()
+__device__ __forceinline__ bool
+group_sync_or(uint32_t group, bool v)
 {
-    return PAIR ? 1u : 2u;
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\n"
+                 "barrier.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(any)
+                 : "r"(group + 1u), "r"((uint32_t)kEdgeThreads), "r"((uint32_t)v)
+                 : "memory");
+    return any != 0u;
 }
 
 template<int K1, bool PAIR, bool SUM>
-__global__ void __launch_bounds__(kEdgeThreads, edge_ctas_per_sm<PAIR>())
+__global__ void __launch_bounds__(kEdgeBlock, 1)
 k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
               const uint32_t* __restrict__ recv, const uint32_t* __restrict__ send,
               const uint16_t* __restrict__ H, uint32_t ldh,
@@ -416,30 +431,36 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
     constexpr uint32_t kW1 = ((64u * K1 * 2u + 1023u) / 1024u) * 1024u;
     constexpr uint32_t kW = 64u * 64u * 2u;            // W2, W3
     constexpr uint32_t kOp = edge_operand_bytes<K1>();
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    // the swizzled operand starts on a 1024-byte boundary
+    uint8_t* smem = smem_raw + ((1024u - (smem_addr(smem_raw) & 1023u)) & 1023u);
+    // layer 1 done, its accumulator read, layers 2 and 3 done
+    __shared__ __align__(8) uint64_t mbars[kEdgeGroups][3];
     __shared__ uint32_t tmem_base;
+    __shared__ __align__(16) float sbias[3][64];
     uint8_t* sW1 = smem;
     uint8_t* sW2 = sW1 + kW1;
     uint8_t* sW3 = sW2 + kW;
-    // an operand buffer holds the layer-1 input (128 x K1), then, once
-    // layer 1's MMAs have completed, the 128 x 64 activations of layers 1
-    // and 2 (and, with SUM, the layer-3 output tile); of the two buffers,
-    // the next tile's input is gathered into the other one while this
-    // tile's layers run
-    constexpr uint32_t kBufs = edge_buffers<PAIR>();
-    uint8_t* const sA0 = sW3 + kW;
-    uint8_t* sA1 = sA0;  // the current tile's buffer
-    EdgeShared* ss = reinterpret_cast<EdgeShared*>(sA0 + kBufs * kOp);
-    const uint32_t tid = threadIdx.x;
+    // the last kEdgeGroups warps gather
+    const bool producer = threadIdx.x >= kEdgeThreads * kEdgeGroups;
+    const uint32_t tid = producer ? threadIdx.x % 32u : threadIdx.x % kEdgeThreads;
+    const uint32_t group = producer ? (threadIdx.x - kEdgeThreads * kEdgeGroups) / 32u
+                                    : threadIdx.x / kEdgeThreads;
     const uint32_t warp = tid >> 5, lane = tid & 31;
+    // the group's buffers: the layer-1 input (128 x K1), free for the next
+    // tile's rows once layer 1's MMAs have completed, and the 128 x 64
+    // activations of layers 1 and 2 (and, with SUM, the layer-3 output tile)
+    uint8_t* const sX = sW3 + kW + group * (kOp + kEdgeAct);
+    uint8_t* const sA1 = sX + kOp;
+    EdgeShared* ss = reinterpret_cast<EdgeShared*>(
+                         sW3 + kW + kEdgeGroups * (kOp + kEdgeAct)) + group;
 
-    for (uint32_t e = tid; e < 64u * K1 / 8u; e += kEdgeThreads) {
+    for (uint32_t e = threadIdx.x; e < 64u * K1 / 8u; e += blockDim.x) {
         const uint32_t row = e / (K1 / 8), g = e % (K1 / 8);
         *reinterpret_cast<uint4*>(sW1 + ((row / 8) * (K1 / 8) + g) * 128 + (row % 8) * 16) =
             *reinterpret_cast<const uint4*>(W1 + (size_t)row * K1 + g * 8);
     }
-    for (uint32_t e = tid; e < 64u * 8u; e += kEdgeThreads) {
+    for (uint32_t e = threadIdx.x; e < 64u * 8u; e += blockDim.x) {
         const uint32_t row = e / 8, g = e % 8;
         const uint32_t o = ((row / 8) * 8 + g) * 128 + (row % 8) * 16;
         *reinterpret_cast<uint4*>(sW2 + o) =
@@ -447,59 +468,90 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
         *reinterpret_cast<uint4*>(sW3 + o) =
             *reinterpret_cast<const uint4*>(W3 + (size_t)row * 64 + g * 8);
     }
-    if (tid < 192)
-        ss->bias[tid / 64][tid % 64] = (tid < 64 ? b1 : (tid < 128 ? b2 : b3))[tid % 64];
-    if (tid == 0)
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" :: "r"(smem_addr(&mbar)));
-    if (warp == 0) {
+    if (threadIdx.x < 192) {
+        const uint32_t t = threadIdx.x;
+        sbias[t / 64][t % 64] = (t < 64 ? b1 : (t < 128 ? b2 : b3))[t % 64];
+    }
+    const uint32_t mbar1 = smem_addr(&mbars[group][0]);
+    const uint32_t mread = smem_addr(&mbars[group][1]);
+    const uint32_t mbar = smem_addr(&mbars[group][2]);
+    if (tid == 0 && !producer) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" :: "r"(mbar1));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n"
+                     :: "r"(mread), "r"((uint32_t)kEdgeWarps));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" :: "r"(mbar));
+        ss->stop = 0;
+    }
+    if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 "
-                     "[%0], %1;\n" :: "r"(smem_addr(&tmem_base)), "r"(64u));
+                     "[%0], %1;\n" :: "r"(smem_addr(&tmem_base)), "r"(kEdgeTmem));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
     }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n");
-    const uint32_t tmem = tmem_base;
+    const uint32_t tmem1 = tmem_base + group * 128u;  // layer 1
+    const uint32_t tmem = tmem1 + 64u;                // layers 2 and 3
     const uint32_t idesc = make_idesc(64);
     uint32_t phase = 0;
     bool failed = false;
 
-    // issue the MMAs of one layer (thread 0) and wait for them (everyone)
+    // one thread issues the MMAs of one layer
+    auto mma = [&](uint32_t acc0, const uint8_t* sA, const uint8_t* sB, uint32_t K,
+                   uint32_t bar) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n");
+        const uint32_t sbo = (K / 8) * 128;
+        for (uint32_t ks = 0; ks < K / 16; ks++) {
+            // the pair input: 64 columns of the receiver and 64 of the sender,
+            // swizzled rows of 128 bytes (K steps of 32 bytes in them), then
+            // the features as core matrices
+            const uint64_t ad =
+                PAIR && K == K1
+                    ? (ks < 8 ? make_desc(smem_addr(sA) + (ks / 4) * 16384u + (ks % 4) * 32u,
+                                          16, 1024) | (2ull << 61)
+                              : make_desc(smem_addr(sA) + 32768u, 128, 256))
+                    : make_desc(smem_addr(sA) + ks * 256, 128, sbo);
+            const uint64_t bd = make_desc(smem_addr(sB) + ks * 256, 128, sbo);
+            const uint32_t acc = ks > 0 ? 1u : 0u;
+            asm volatile(
+                "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                :: "r"(acc0), "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one."
+                     "shared::cluster.b64 [%0];\n" :: "r"(bar));
+    };
+    auto arrived = [&](uint32_t bar, uint32_t parity) {
+        uint32_t done;
+        asm volatile("{\n.reg .pred p;\n"
+                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                     "selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done) : "r"(bar), "r"(parity));
+        return done != 0u;
+    };
     bool tile_bad = false;
-    auto layer = [&](const uint8_t* sA, const uint8_t* sB, uint32_t K) {
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;\n");
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n");
-            const uint32_t sbo = (K / 8) * 128;
-            for (uint32_t ks = 0; ks < K / 16; ks++) {
-                const uint64_t ad = make_desc(smem_addr(sA) + ks * 256, 128, sbo);
-                const uint64_t bd = make_desc(smem_addr(sB) + ks * 256, 128, sbo);
-                const uint32_t acc = ks > 0 ? 1u : 0u;
-                asm volatile(
-                    "{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                    :: "r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one."
-                         "shared::cluster.b64 [%0];\n" :: "r"(smem_addr(&mbar)));
-        }
-        uint32_t done = 0;
-        for (uint32_t it = 0; it < kWaitLimit && !done; it++) {
-            asm volatile("{\n.reg .pred p;\n"
-                         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                         "selp.u32 %0, 1, 0, p;\n}\n"
-                         : "=r"(done) : "r"(smem_addr(&mbar)), "r"(phase));
-        }
+    auto wait = [&](uint32_t bar, uint32_t parity) {
+        bool done = false;
+        for (uint32_t it = 0; it < kWaitLimit && !done; it++)
+            done = arrived(bar, parity);
         // a time-out is recorded and acted on at the end of the tile (one
-        // CTA-wide vote per tile instead of one per layer)
+        // group-wide vote per tile instead of one per layer)
         const bool bad = !__all_sync(0xffffffffu, done) || fake != 0u;
         if (bad && lane == 0)
             atomicExch(err, 1);
         tile_bad = tile_bad || bad;
-        phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;\n");
+    };
+    // layers 2 and 3: thread 0 issues, everyone waits
+    auto layer = [&](const uint8_t* sB) {
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n");
+        group_sync(group);
+        if (tid == 0)
+            mma(tmem, sA1, sB, 64, mbar);
+        wait(mbar, phase);
+        phase ^= 1u;
     };
     // this thread's row of the accumulator and half of its columns
     const uint32_t row = (warp & 3u) * 32u + lane;
@@ -507,7 +559,8 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
     // read the accumulator (32 columns), add the bias, activate;
     // `emit(g, packed8)` receives the row's k-group g (8 bf16 as a uint4)
     auto epilogue = [&](int layer_index, int act, auto&& emit) {
-        const uint32_t taddr = tmem + (((warp & 3u) * 32u) << 16) + half * 32u;
+        const uint32_t taddr = (layer_index == 0 ? tmem1 : tmem) +
+                               (((warp & 3u) * 32u) << 16) + half * 32u;
         uint32_t v[32];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -522,7 +575,14 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
               "=r"(v[30]), "=r"(v[31])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;\n");
-        const float* bias = ss->bias[layer_index] + half * 32u;
+        if (layer_index == 0) {  // the next tile's layer 1 may overwrite it
+            asm volatile("tcgen05.fence::before_thread_sync;\n");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" :: "r"(mread)
+                             : "memory");
+        }
+        const float* bias = sbias[layer_index] + half * 32u;
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             uint32_t p[4];
@@ -542,11 +602,13 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
         *reinterpret_cast<uint4*>(sA1 + ((row / 8) * 8 + g) * 128 + (row % 8) * 16) = val;
     };
 
-    // the edges of this CTA: every tile (grid-stride), or, with SUM, the
-    // edges of its receivers
+    // the edges of this group: every tile (grid-stride), or, with SUM, the
+    // edges of its receivers; few tiles go to one group of each CTA first
+    const uint32_t groups = gridDim.x * kEdgeGroups;
+    const uint32_t me = group * gridDim.x + blockIdx.x;
     uint32_t e_begin = 0, e_end = E;
     if constexpr (SUM) {
-        if (tid == 0) {
+        if (tid == 0 && !producer) {
             // first node s in [0, n_nodes] with off[s] >= v
             auto lower = [&](uint64_t v) -> uint32_t {
                 uint32_t lo = 0, hi = n_nodes;
@@ -559,17 +621,16 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
                 }
                 return lo;
             };
-            const uint64_t G = gridDim.x;
-            ss->nodes[0] = blockIdx.x == 0 ? 0u : lower((uint64_t)blockIdx.x * E / G);
-            ss->nodes[1] = blockIdx.x + 1 == gridDim.x
-                               ? n_nodes
-                               : lower((uint64_t)(blockIdx.x + 1) * E / G);
+            const uint64_t G = groups;
+            ss->nodes[0] = me == 0 ? 0u : lower((uint64_t)me * E / G);
+            ss->nodes[1] = me + 1 == groups ? n_nodes
+                                            : lower((uint64_t)(me + 1) * E / G);
             ss->carry_node[0] = ss->carry_node[1] = 0xffffffffu;
         }
         __syncthreads();
         const uint32_t n_lo = ss->nodes[0], n_hi = ss->nodes[1];
         // receivers without edges: a zero sum
-        for (uint32_t s = n_lo + tid; s < n_hi; s += kEdgeThreads)
+        for (uint32_t s = n_lo + tid; s < n_hi && !producer; s += kEdgeThreads)
             if (off[s] == off[s + 1]) {
                 uint4* dst = reinterpret_cast<uint4*>(Y + (size_t)s * ldy + col);
                 for (int g = 0; g < 8; g++)
@@ -580,86 +641,96 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
     }
     const uint32_t tiles = SUM ? (e_end - e_begin + kTcRows - 1) / kTcRows
                                : (E + kTcRows - 1) / kTcRows;
-    // the edge indices of tile t's rows, loaded one tile ahead: the
-    // receiver (threads of the first part; ~0 past the last edge) and the
-    // sender (pair input)
-    constexpr uint32_t kg = K1 / 8;
-    const uint32_t grow = tid % kTcRows, part = tid / kTcRows;
-    auto load_idx = [&](uint32_t t, uint32_t& ei, uint32_t& es) {
-        ei = 0xffffffffu;
-        es = 0u;
-        if (t >= tiles)
-            return;
-        const uint32_t e = e_begin + t * kTcRows + grow;
-        if (e >= e_end)
-            return;
-        if ((PAIR || SUM) && part == 0)
-            ei = recv[e];
-        if (PAIR)
-            es = send[e];
-    };
-    // gathers the layer-1 input of tile t into buf: thread t copies k-groups
-    // [part * kg / 2, (part + 1) * kg / 2) of row t % 128 (asynchronous
-    // copies, committed by the caller)
-    auto gather = [&](uint32_t t, uint8_t* buf, uint32_t ei, uint32_t es) {
-        const uint32_t e = e_begin + t * kTcRows + grow;
-        const bool valid = e < e_end;
-        uint8_t* row0 = buf + (grow / 8) * kg * 128 + (grow % 8) * 16;
-        const uint32_t g0 = part * (kg / 2), g1 = g0 + kg / 2;
-        if (PAIR) {
-            const uint32_t eiv = (valid && part == 0) ? ei : 0u;
-            const uint32_t esv = valid ? es : 0u;
-            for (uint32_t g = g0; g < g1; g++) {
-                const uint16_t* src =
-                    g < 8 ? H + (size_t)eiv * ldh + g * 8
-                          : (g < 16 ? H + (size_t)esv * ldh + (g - 8) * 8
-                                    : Ef + (size_t)(valid ? e : 0u) * 16 + (g - 16) * 8);
-                cp_async_16z(row0 + g * 128, src, valid);
+    const uint32_t stride = SUM ? 1u : groups;
+    uint32_t tile = SUM ? 0u : me;
+    if (producer) {
+        // rows of 32 bytes and multiples (X, the features): a lane copies every
+        // other k-group of 8 rows, so that a copy instruction of the warp reads
+        // whole 32-byte sectors.  Node rows of 128 bytes: eight lanes a row,
+        // and swizzled rows in shared memory, so that a line that arrives is
+        // written at once: as core matrices its pieces fall into the same
+        // banks, and the epilogues' own accesses waited for them (an epilogue
+        // was 3,900 cycles instead of 1,400)
+        constexpr uint32_t kg = PAIR ? 2 : K1 / 8;
+        const uint32_t r0 = (lane & 7u) + ((lane >> 4) << 3), gh = (lane >> 3) & 1u;
+        uint32_t ei[4], es[4];  // receivers and senders of rows lane, lane + 32, ..
+        auto load_idx = [&](uint32_t t) {
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++) {
+                const uint32_t e = e_begin + t * kTcRows + q * 32u + lane;
+                const bool valid = PAIR && t < tiles && e < e_end;
+                ei[q] = valid ? recv[e] : 0u;
+                es[q] = valid ? send[e] : 0u;
             }
-        } else {
-            for (uint32_t g = g0; g < g1; g++)
-                cp_async_16z(row0 + g * 128, X + (size_t)(valid ? e : 0u) * ldx + g * 8,
-                             valid);
+        };
+        load_idx(tile);
+        for (uint32_t n = 0; tile < tiles; n++, tile += stride) {
+            const uint32_t e0 = e_begin + tile * kTcRows;
+            if (PAIR) {
+                const uint32_t c = lane & 7u, rl = lane >> 3;
+#pragma unroll
+                for (uint32_t j = 0; j < 32; j++) {
+                    const uint32_t row = j * 4u + rl;
+                    const bool valid = e0 + row < e_end;
+                    const uint32_t from = (j & 7u) * 4u + rl;
+                    const uint32_t vr = __shfl_sync(0xffffffffu, ei[j / 8], from);
+                    const uint32_t vs = __shfl_sync(0xffffffffu, es[j / 8], from);
+                    uint8_t* dst = sX + row * 128u + ((c ^ (row & 7u)) << 4);
+                    cp_async_16z(dst, H + (size_t)vr * ldh + c * 8, valid);
+                    cp_async_16z(dst + 16384, H + (size_t)vs * ldh + c * 8, valid);
+                }
+            }
+            const uint16_t* src = PAIR ? Ef : X;
+            const uint32_t ld = PAIR ? 16u : ldx;
+#pragma unroll
+            for (uint32_t j = 0; j < 8; j++) {
+                const uint32_t row = j * 16u + r0;
+                const bool valid = e0 + row < e_end;
+                const size_t ev = valid ? e0 + row : 0u;
+                uint8_t* dst = sX + (PAIR ? 32768u : 0u) + (row / 8) * kg * 128 +
+                               (row % 8) * 16 + gh * 128;
+#pragma unroll
+                for (uint32_t g = 0; g < kg; g += 2)
+                    cp_async_16z(dst + g * 128, src + ev * ld + (g + gh) * 8, valid);
+            }
+            load_idx(tile + stride);
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            // the accumulator of the tile before has been read
+            bool ok = n == 0;
+            for (uint32_t it = 0; it < kWaitLimit && !ok; it++) {
+                ok = arrived(mread, (n - 1u) & 1u);
+                if (!ok && *(volatile uint32_t*)&ss->stop)
+                    break;
+            }
+            if (!__all_sync(0xffffffffu, ok))
+                break;
+            if (lane == 0)
+                mma(tmem1, sX, sW1, K1, mbar1);
+            wait(mbar1, n & 1u);  // the operand buffer is free
+            if (tile_bad)
+                break;
         }
+    }
+    // the receiver of row tid of tile t, loaded one tile ahead (~0 past the
+    // last edge)
+    auto load_recv = [&](uint32_t t) {
+        const uint32_t e = e_begin + t * kTcRows + tid;
+        return SUM && tid < kTcRows && t < tiles && e < e_end ? recv[e] : 0xffffffffu;
     };
-    const uint32_t stride = SUM ? 1u : gridDim.x;
-    uint32_t tile = SUM ? 0u : blockIdx.x;
-    uint32_t ei_cur, es_cur;
-    load_idx(tile, ei_cur, es_cur);
-    uint32_t cur = 0;
-    if (kBufs == 2 && tile < tiles)
-        gather(tile, sA0, ei_cur, es_cur);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    for (; tile < tiles && !failed; tile += stride) {
-        const uint32_t next = tile + stride;
-        uint32_t ei_next, es_next;
-        load_idx(next, ei_next, es_next);
-        if constexpr (kBufs == 2) {
-            // the next tile's gather overlaps this tile's layers
-            if (next < tiles)
-                gather(next, sA0 + (cur ^ 1u) * kOp, ei_next, es_next);
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        } else {
-            gather(tile, sA0, ei_cur, es_cur);
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
+    uint32_t ei_cur = producer ? 0u : load_recv(tile);
+    for (uint32_t n = 0; !producer && tile < tiles && !failed; n++, tile += stride) {
+        const uint32_t ei_next = load_recv(tile + stride);
         const uint32_t eb = e_begin + tile * kTcRows;
         const uint32_t e = eb + row;
         const bool valid = e < e_end;
-        sA1 = sA0 + cur * kOp;
-        if (SUM && part == 0)
-            ss->recv[grow] = ei_cur;
-        // the receiver of the edge after this tile's (~0 at the end of the
-        // CTA's edges): it tells whether the tile's last run is complete
-        if (SUM && tid == 0)
-            ss->next_recv = ei_next;
-        layer(sA1, sW1, K1);
+        if (SUM && tid < kTcRows)
+            ss->recv[tid] = ei_cur;
+        wait(mbar1, n & 1u);
         epilogue(0, act1, to_a1);
-        layer(sA1, sW2, 64);
+        layer(sW2);
         epilogue(1, act2, to_a1);
-        layer(sA1, sW3, 64);
+        layer(sW3);
         if constexpr (!SUM) {
             epilogue(2, act3, [&](int g, uint4 val) {
                 if (valid)
@@ -671,6 +742,10 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
             epilogue(2, act3, [&](int g, uint4 val) {
                 *reinterpret_cast<uint4*>(sA1 + row * 128u + ((g ^ (row & 7u)) * 16u)) = val;
             });
+            // the receiver of the edge after this tile's (~0 at the end of the
+            // group's edges): it tells whether the tile's last run is complete
+            if (tid == 0)
+                ss->next_recv = ei_next;
             const uint32_t nvalid = min((uint32_t)kTcRows, e_end - eb);
             if (warp < 4) {
                 const uint32_t rr = warp * 32u + lane;
@@ -679,8 +754,11 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
                 if (lane == 0)
                     ss->start[warp] = bal;
             }
-            __syncthreads();
+            group_sync(group);
             const uint32_t par = tile & 1u;
+            // run k of the tile: warp k % 8, two columns a lane
+            const uint32_t cg = (lane >> 2) << 4;
+            const uint8_t* sc = sA1 + (lane & 3u) * 4u;
             uint32_t ord = 0;
             for (uint32_t wq = 0; wq < 4; wq++) {
                 uint32_t m = ss->start[wq];
@@ -703,64 +781,68 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
                         }
                     }
                     const uint32_t node = ss->recv[a];
-                    float a0 = 0.f, a1 = 0.f;
+                    float s0 = 0.f, s1 = 0.f;  // columns 2 lane, 2 lane + 1
                     if (a == 0 && ss->carry_node[par] == node) {
-                        a0 = ss->carry[par][2 * lane];
-                        a1 = ss->carry[par][2 * lane + 1];
+                        s0 = ss->carry[par][2 * lane];
+                        s1 = ss->carry[par][2 * lane + 1];
                     }
-                    // row k's two columns of this lane
-                    auto ld_row = [&](uint32_t k) -> uint32_t {
-                        return *reinterpret_cast<const uint32_t*>(
-                            sA1 + k * 128u + (((lane >> 2) ^ (k & 7u)) * 16u) +
-                            (lane & 3u) * 4u);
-                    };
-                    // eight loads in flight, then the additions in row order
-                    uint32_t k = a;
-                    for (; k + 8u <= b; k += 8u) {
-                        uint32_t v[8];
+                    // eight loads in flight, then the additions in row order;
+                    // the swizzle is the same for rows eight apart
+                    uint32_t o[8];
 #pragma unroll
-                        for (int u = 0; u < 8; u++)
-                            v[u] = ld_row(k + u);
+                    for (uint32_t u = 0; u < 8; u++)
+                        o[u] = u * 128u + (cg ^ (((a + u) & 7u) << 4));
+                    const uint8_t* q = sc + a * 128u;
+                    uint32_t left = b - a, v[8];
+                    for (; left >= 8u; left -= 8u, q += 1024) {
 #pragma unroll
-                        for (int u = 0; u < 8; u++) {
-                            a0 += __uint_as_float(v[u] << 16);
-                            a1 += __uint_as_float(v[u] & 0xffff0000u);
+                        for (uint32_t u = 0; u < 8; u++)
+                            v[u] = *reinterpret_cast<const uint32_t*>(q + o[u]);
+#pragma unroll
+                        for (uint32_t u = 0; u < 8; u++) {
+                            s0 += __uint_as_float(v[u] << 16);
+                            s1 += __uint_as_float(v[u] & 0xffff0000u);
                         }
                     }
-                    for (; k < b; k++) {
-                        const uint32_t v = ld_row(k);
-                        a0 += __uint_as_float(v << 16);
-                        a1 += __uint_as_float(v & 0xffff0000u);
-                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < 7; u++)
+                        if (u < left)
+                            v[u] = *reinterpret_cast<const uint32_t*>(q + o[u]);
+#pragma unroll
+                    for (uint32_t u = 0; u < 7; u++)
+                        if (u < left) {
+                            s0 += __uint_as_float(v[u] << 16);
+                            s1 += __uint_as_float(v[u] & 0xffff0000u);
+                        }
                     if (b < nvalid || ss->next_recv != node) {
-                        *reinterpret_cast<uint32_t*>(Y + (size_t)node * ldy + col +
-                                                     2 * lane) =
-                            pack2(a0 * scale, a1 * scale);
+                        *reinterpret_cast<uint32_t*>(Y + (size_t)node * ldy + col + 2 * lane) =
+                            pack2(s0 * scale, s1 * scale);
                     } else {
                         // the last run: its receiver continues in the next tile
-                        ss->carry[par ^ 1u][2 * lane] = a0;
-                        ss->carry[par ^ 1u][2 * lane + 1] = a1;
+                        ss->carry[par ^ 1u][2 * lane] = s0;
+                        ss->carry[par ^ 1u][2 * lane + 1] = s1;
                         if (lane == 0)
                             ss->carry_node[par ^ 1u] = node;
                     }
                 }
             }
         }
-        // the tile after next reuses this buffer; the next tile's MMAs
-        // reuse the accumulator; a time-out in any layer ends the CTA
+        // the next tile reuses the activations and the accumulator; a
+        // time-out in any layer ends the group
         asm volatile("tcgen05.fence::before_thread_sync;\n");
-        failed = __syncthreads_or(tile_bad);
+        failed = group_sync_or(group, tile_bad);
         ei_cur = ei_next;
-        es_cur = es_next;
-        cur = (cur + 1u) % kBufs;
+        if (failed && tid == 0)
+            *(volatile uint32_t*)&ss->stop = 1u;
     }
     // no copy may still be in flight when the CTA ends (after a time-out)
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
     __syncthreads();
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         asm volatile("tcgen05.fence::after_thread_sync;\n");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n"
-                     :: "r"(tmem), "r"(64u));
+                     :: "r"(tmem_base), "r"(kEdgeTmem));
     }
 }
 
@@ -769,15 +851,9 @@ constexpr size_t
 edge_mlp_smem()
 {
     return ((64u * K1 * 2u + 1023u) / 1024u) * 1024u + 2u * 64u * 64u * 2u +
-           edge_buffers<K1 == 144>() * edge_operand_bytes<K1>() + sizeof(EdgeShared);
+           kEdgeGroups * (edge_operand_bytes<K1>() + kEdgeAct + sizeof(EdgeShared)) + 1024u;
 }
-static_assert(edge_ctas_per_sm<true>() * (edge_mlp_smem<144>() + 1024) <= 228 * 1024,
-              "pair-input CTAs per SM");
-static_assert(edge_ctas_per_sm<false>() * (edge_mlp_smem<16>() + 1024) <= 228 * 1024,
-              "row-input CTAs per SM");
-static_assert(edge_ctas_per_sm<false>() * (edge_mlp_smem<80>() + 1024) <= 228 * 1024,
-              "80-wide row-input CTAs per SM");
-
+static_assert(edge_mlp_smem<144>() <= 226 * 1024, "one CTA per SM");
 
 // ---------------------------------------------------------------------------
 // Backward of a dense layer on the tensor cores (training).
@@ -1223,30 +1299,24 @@ aqua_gnn_edge_mlp_tc(uint32_t E, uint32_t K1, const uint16_t* X, uint32_t ldx,
     const aqua_status st = edge_mlp_configure(sms);
     if (st != AQUA_OK)
         return st;
+    // one CTA per SM (shared memory; 192 of the 512 TMEM columns)
     const uint32_t tiles = (E + kTcRows - 1) / kTcRows;
+    const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
     cudaStream_t s = (cudaStream_t)stream;
     if (pair) {
-        // 72 KB of shared memory: three CTAs per SM (192 of 512 TMEM columns)
-        const uint32_t cap = (uint32_t)sms * edge_ctas_per_sm<true>();
-        const uint32_t grid = tiles < cap ? tiles : cap;
         k_edge_mlp_tc<144, true, false>
-            <<<grid, kEdgeThreads, edge_mlp_smem<144>(), s>>>(
+            <<<grid, kEdgeBlock, edge_mlp_smem<144>(), s>>>(
                 E, nullptr, 0, recv, send, H, ldh, Ef, W1, b1, W2, b2, W3, b3,
                 act1, act2, act3, Y, ldy, err, (uint32_t)aqua::g_debug_fake_timeout, 0u, nullptr, 0.f, 0u);
     } else if (K1 == 80) {
-        // the first node MLP, n1 (80-wide rows): 70 KB, three CTAs per SM
-        const uint32_t cap = (uint32_t)sms * edge_ctas_per_sm<false>();
-        const uint32_t grid = tiles < cap ? tiles : cap;
+        // the first node MLP, n1 (80-wide rows)
         k_edge_mlp_tc<80, false, false>
-            <<<grid, kEdgeThreads, edge_mlp_smem<80>(), s>>>(
+            <<<grid, kEdgeBlock, edge_mlp_smem<80>(), s>>>(
                 E, X, ldx, nullptr, nullptr, nullptr, 0, nullptr, W1, b1, W2,
                 b2, W3, b3, act1, act2, act3, Y, ldy, err, (uint32_t)aqua::g_debug_fake_timeout, 0u, nullptr, 0.f, 0u);
     } else {
-        // 52 KB: three CTAs per SM (registers; 192 TMEM columns)
-        const uint32_t cap = (uint32_t)sms * edge_ctas_per_sm<false>();
-        const uint32_t grid = tiles < cap ? tiles : cap;
         k_edge_mlp_tc<16, false, false>
-            <<<grid, kEdgeThreads, edge_mlp_smem<16>(), s>>>(
+            <<<grid, kEdgeBlock, edge_mlp_smem<16>(), s>>>(
                 E, X, ldx, nullptr, nullptr, nullptr, 0, nullptr, W1, b1, W2,
                 b2, W3, b3, act1, act2, act3, Y, ldy, err, (uint32_t)aqua::g_debug_fake_timeout, 0u, nullptr, 0.f, 0u);
     }
@@ -1277,23 +1347,22 @@ aqua_gnn_edge_mlp_sum_tc(uint32_t n_nodes, uint32_t E, uint32_t K1,
     const aqua_status st = edge_mlp_configure(sms);
     if (st != AQUA_OK)
         return st;
-    // each CTA owns the receivers of about E / grid edges; a small graph
-    // gets fewer CTAs (at least one, for the receivers without edges)
+    // each group of a CTA owns the receivers of about E / groups edges; a
+    // small graph gets fewer CTAs (at least one, for the receivers without
+    // edges)
     const uint32_t tiles = (E + kTcRows - 1) / kTcRows;
-    const uint32_t per_sm = (uint32_t)(pair ? edge_ctas_per_sm<true>()
-                                             : edge_ctas_per_sm<false>());
-    uint32_t grid = (uint32_t)sms * per_sm;
+    uint32_t grid = (uint32_t)sms;
     if (tiles < grid)
         grid = tiles > 0 ? tiles : 1u;
     cudaStream_t s = (cudaStream_t)stream;
     if (pair)
         k_edge_mlp_tc<144, true, true>
-            <<<grid, kEdgeThreads, edge_mlp_smem<144>(), s>>>(
+            <<<grid, kEdgeBlock, edge_mlp_smem<144>(), s>>>(
                 E, nullptr, 0, recv, send, H, ldh, Ef, W1, b1, W2, b2, W3, b3,
                 act1, act2, act3, out, ld, err, (uint32_t)aqua::g_debug_fake_timeout, n_nodes, offsets, scale, col);
     else
         k_edge_mlp_tc<16, false, true>
-            <<<grid, kEdgeThreads, edge_mlp_smem<16>(), s>>>(
+            <<<grid, kEdgeBlock, edge_mlp_smem<16>(), s>>>(
                 E, X, ldx, recv, nullptr, nullptr, 0, nullptr, W1, b1, W2, b2,
                 W3, b3, act1, act2, act3, out, ld, err, (uint32_t)aqua::g_debug_fake_timeout, n_nodes, offsets, scale,
                 col);

@@ -324,16 +324,16 @@ k_linear_fwd_tc(uint32_t M, uint32_t K, const uint16_t* __restrict__ X,
 // ---------------------------------------------------------------------------
 // Fused three-layer edge MLP: Y = L3(act(L2(act(L1(X))))) on tiles of 128
 // edges, every activation kept on chip.  The layer-1 input of each tile is
-// gathered into shared memory by asynchronous copies: rows of X, or, in PAIR mode, the concatenation [H[recv[e]] (64),
-// H[send[e]] (64), Ef[e] (16)] that aqua_gnn_gather_pair materialises.  The
-// layers accumulate in 64 columns of tensor memory (layer 1 in its own, layers 2
-// and 3 in turn); each epilogue reads them back (tcgen05.ld), adds the bias, applies the activation, rounds
-// to BF16 and writes the next layer's A operand into shared memory, exactly
-// the values the unfused layers store to and reload from global memory, so
-// the result is bit-identical to three aqua_gnn_linear_fwd_tc calls.  Only
-// the BF16 output of layer 3 is written.  A wait that times out sets *err;
-// the group finishes that tile (its outputs are then not to be trusted) and
-// stops.
+// gathered into shared memory by asynchronous copies: rows of X, or, in PAIR
+// mode, the concatenation [H[recv[e]] (64), H[send[e]] (64), Ef[e] (16)] that
+// aqua_gnn_gather_pair materialises.  The layers accumulate in 64 columns of
+// tensor memory (layer 1 in its own, layers 2 and 3 in turn); each epilogue
+// reads them back (tcgen05.ld), adds the bias, applies the activation, rounds
+// to BF16 and writes the next layer's A operand into shared memory, exactly the
+// values the unfused layers store to and reload from global memory, so the
+// result is bit-identical to three aqua_gnn_linear_fwd_tc calls.  Only the BF16
+// output of layer 3 is written.  A wait that times out sets *err; the group
+// finishes that tile (its outputs are then not to be trusted) and stops.
 //
 // The tile's chain of layers, barriers and sums bounds it, not the tensor pipe
 // (10%) nor memory: three groups a CTA run three chains, and a warp of each

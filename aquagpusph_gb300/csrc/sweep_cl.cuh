@@ -400,6 +400,12 @@ k_sweep_cl(Consts c, StepArgs a)
         else if (c.debug_fake_timeout)
             ok = false;  // test switch: the copies have completed
         parity ^= 1u;
+        // zero records up to the next multiple of 64, so that the scan tests
+        // no bounds
+        const uint32_t n = min(S.total - p * (uint32_t)CAP, (uint32_t)CAP);
+        if (n + tid < ((n + 63u) & ~63u))
+            S.r0[n + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncthreads();  // S.piece / S.nstaged visible; the vote below
         const bool bad = __syncthreads_or(!ok);
         if (bad) {
@@ -650,20 +656,20 @@ k_sweep_cl(Consts c, StepArgs a)
                     uint32_t fill = 0;
                     uint32_t wdone = wfill;  // wall entries already summed
                     const uint32_t g = part ? u % share : 0u, G = part ? share : 1u;
-                    const uint32_t k_end = nst * (g + 1u) / G;
+                    const uint32_t rounds = (nst + 63u) / 64u;
+                    const uint32_t k_end = rounds * (g + 1u) / G * 64u;
                     // 64 records per round, two per lane, listed in staging
                     // order
-                    for (uint32_t base = nst * g / G; base < k_end; base += 64) {
+                    for (uint32_t base = rounds * g / G * 64u; base < k_end; base += 64) {
                         unsigned bf[2], bw[2];
                         bool fl[2], wa[2];
 #pragma unroll
                         for (int v = 0; v < 2; v++) {
-                            const uint32_t k = base + 32u * v + lane;
-                            const float4 r = S.r0[min(k, (uint32_t)CAP)];
+                            const float4 r = S.r0[base + 32u * v + lane];
                             const float dx = fmaxf(fmaxf(lo[0] - r.x, r.x - hi[0]), 0.f);
                             const float dy = fmaxf(fmaxf(lo[1] - r.y, r.y - hi[1]), 0.f);
                             const float dz = fmaxf(fmaxf(lo[2] - r.z, r.z - hi[2]), 0.f);
-                            const bool in = k < k_end && dx * dx + dy * dy + dz * dz < R2;
+                            const bool in = dx * dx + dy * dy + dz * dz < R2;
                             fl[v] = in && r.w > 0.f;
                             // the boundary elements matter to fluid only
                             wa[v] = in && r.w < 0.f && any_fluid;

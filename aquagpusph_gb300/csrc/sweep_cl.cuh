@@ -33,6 +33,12 @@
 // lattice most cells hold 9 clusters, and seven warps would wait for the
 // ninth.
 //
+// Instruction issue bounds it (72% of the slots, 24 warps an SM by shared
+// memory).  Clusters by octant, with one mask per staged record for all eight,
+// were 5 to 7 of 8 full off the lattice: 5.9M sheared particles 9.39 ms a call,
+// now 8.2; 406,402: 1.09 ms, now 0.80.  On a lattice at rest octants are perfect
+// clusters, and those masks were 9% cheaper (5.88M: 5.75 ms a step, now 6.28).
+//
 // Boundary elements reach fluid particles through a second list (the BIe
 // wall sums), which also serves the elastic bounce and PST of the
 // epilogue.  Where that list overflowed or the neighbourhood needed more
@@ -661,7 +667,7 @@ k_sweep_cl(Consts c, StepArgs a)
                     // 64 records per round, two per lane, listed in staging
                     // order
                     for (uint32_t base = rounds * g / G * 64u; base < k_end; base += 64) {
-                        unsigned bf[2], bw[2];
+                        unsigned bf[2];
                         bool fl[2], wa[2];
 #pragma unroll
                         for (int v = 0; v < 2; v++) {
@@ -674,17 +680,17 @@ k_sweep_cl(Consts c, StepArgs a)
                             // the boundary elements matter to fluid only
                             wa[v] = in && r.w < 0.f && any_fluid;
                             bf[v] = __ballot_sync(0xffffffffu, fl[v]);
-                            bw[v] = __ballot_sync(0xffffffffu, wa[v]);
                         }
-                        uint32_t wtot = bw[0] | bw[1], wbefore = 0;
                         if (fl[0])
                             list[fill + (uint32_t)__popc(bf[0] & lt)] = (uint16_t)(base + lane);
                         fill += (uint32_t)__popc(bf[0]);
                         if (fl[1])
                             list[fill + (uint32_t)__popc(bf[1] & lt)] = (uint16_t)(base + 32u + lane);
                         fill += (uint32_t)__popc(bf[1]);
-                        if (wtot) {
-                            wtot = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1]);
+                        if (__any_sync(0xffffffffu, wa[0] || wa[1])) {
+                            const unsigned bw[2] = { __ballot_sync(0xffffffffu, wa[0]),
+                                                     __ballot_sync(0xffffffffu, wa[1]) };
+                            const uint32_t wtot = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1]);
                             if (wfill + wtot > (uint32_t)kClWallCap) {
                                 // the wall list is full: sum it, and let the
                                 // epilogue walk the walls from global memory
@@ -699,7 +705,7 @@ k_sweep_cl(Consts c, StepArgs a)
                                 wdone = 0;
                                 walls_global = true;
                             }
-                            wbefore = (uint32_t)__popc(bw[0] & lt);
+                            uint32_t wbefore = (uint32_t)__popc(bw[0] & lt);
                             if (wa[0])
                                 wl[wfill + wbefore] = (uint16_t)(base + lane);
                             wbefore = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1] & lt);

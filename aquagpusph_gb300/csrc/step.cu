@@ -89,9 +89,9 @@ __constant__ uint8_t kHilbert2[64] = {
 // CELLS = true (clustered sweep, 3-D): the work list holds cells (work, wcl);
 // a cell's clusters take the slots of clu from its first sorted index on, the
 // boundary elements and then the probes come last, in clusters of their own
-// (mixed with the elements the fluid's clusters lose their compact boxes: 1.9M
-// particles at rest on a lattice 6% slower, 5.9M off it 1.4%), and crow holds the
-// cell's neighbourhood as 9 rows of 3 cells.
+// (mixed with the elements the fluid's clusters lose their compact boxes: a
+// 5.88M step on a lattice took 6.73 ms, then 6.52, and a 5.9M call off it 8.57,
+// then 8.45), and crow holds the cell's neighbourhood as 9 rows of 3 cells.
 constexpr int kClusterThreads = 256;
 template<int D, bool CELLS>
 __global__ void __launch_bounds__(kClusterThreads)

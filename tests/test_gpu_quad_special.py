@@ -1,0 +1,44 @@
+"""The quad sweep beside the direct sweep of a thread per particle (the same
+sums in the same order, by plain expressions): equal bit for bit where values
+are not finite or zero."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from test_gpu_quad import cloud
+
+
+def step(c, variant, blocks):
+    from aquagpusph_gb300.solver import Solver
+    sv = Solver(c.params, capacity=c.N)
+    sv.set_tuning(variant, blocks)
+    sv.set_case(c)
+    sv.step(1, graph=True)
+    g = sv.get_case()
+    sv.close()
+    return g
+
+
+def assert_same(c):
+    a, b = step(c, 16, 3), step(c, 9, 14)
+    for name, x in a.state_arrays().items():
+        assert np.array_equal(x, getattr(b, name), equal_nan=x.dtype.kind == "f"), name
+    assert np.array_equal(a.shepard, b.shepard, equal_nan=True)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("n,spread", [(1, 0.2), (5, 0.5), (60, 0.9)])
+@pytest.mark.parametrize("name,value", [
+    ("u", np.inf), ("u", -np.inf), ("u", np.nan), ("u", 3e38), ("dudt", np.inf),
+    ("rho", np.inf), ("rho", np.nan), ("rho", 0.0), ("m", np.inf), ("m", np.nan), ("m", 0.0)])
+def test_values_that_are_not_finite(dims, n, spread, name, value):
+    """One fluid particle with such a value, alone (with slots that hold no
+    neighbour) and among others."""
+    c = cloud(dims, n, spread, 31 * n + dims, 8)
+    a = getattr(c, name)
+    if a.ndim == 2:
+        a[n // 2, 0] = value
+    else:
+        a[n // 2] = value
+    assert_same(c)

@@ -18,6 +18,7 @@
 #include <cstdint>
 
 #include "aqua_learned.h"
+#include "arith.cuh"
 
 namespace aqua {
 // test-only switch of aqua_debug_fake_timeouts() (api.cu)
@@ -873,21 +874,6 @@ static_assert(edge_mlp_smem<144>() <= 226 * 1024, "one CTA per SM");
 // of dY (db).  At the end each CTA adds its partial dW, db to the outputs
 // with atomics.
 
-__device__ __forceinline__ float
-silu_grad_f(float z)
-{
-    // 1 / b by two Newton steps, free of branches up to b = 2^100: the IEEE
-    // reciprocal but for about one value in 5e7 (one ulp)
-    const float b = 1.f + __expf(-z);
-    float s;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(b));
-    s = __fmaf_rn(s, __fmaf_rn(-b, s, 1.f), s);
-    s = __fmaf_rn(s, __fmaf_rn(-b, s, 1.f), s);
-    if (b > 0x1p100f)
-        s = 1.f / b;
-    return s * (1.f + z * (1.f - s));
-}
-
 // bounded wait for a commit on `mbar` (phase parity `phase`); every thread
 // of the CTA returns the same verdict
 __device__ __forceinline__ bool
@@ -1018,10 +1004,10 @@ k_linear_dgrad_tc(uint32_t M, uint32_t N, uint32_t K,
                     for (int j = 0; j < 16; j += 4) {
                         const float4 zz = *reinterpret_cast<const float4*>(
                             warp_chunk(wbuf, lane, 4 * h + j / 4));
-                        d[j] *= silu_grad_f(zz.x);
-                        d[j + 1] *= silu_grad_f(zz.y);
-                        d[j + 2] *= silu_grad_f(zz.z);
-                        d[j + 3] *= silu_grad_f(zz.w);
+                        d[j] *= aqua::silu_grad_f(zz.x);
+                        d[j + 1] *= aqua::silu_grad_f(zz.y);
+                        d[j + 2] *= aqua::silu_grad_f(zz.z);
+                        d[j + 3] *= aqua::silu_grad_f(zz.w);
                     }
                 }
                 for (int j = 0; j < 8; j++)

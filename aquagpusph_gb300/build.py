@@ -90,7 +90,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objdir = os.path.join(ROOT, "_build", "aqua_gb300")
     os.makedirs(objdir, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC)
-               if f.endswith((".cuh", ".h"))]
+               if f.endswith((".cuh", ".h", ".hpp"))]
     headers.append(os.path.join(ROOT, "include", "aqua_gb300.h"))
     cc = nvcc()
     jobs = []

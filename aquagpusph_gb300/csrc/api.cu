@@ -12,6 +12,7 @@
 #include <new>
 
 #include "aqua_internal.cuh"
+#include "copy_route.hpp"
 #include "kernels.cuh"
 
 using namespace aqua;
@@ -440,9 +441,8 @@ enqueue_step(aqua_ctx* x, int cur, cudaStream_t s)
 
 // Field copies of a state.  Between device arrays of this context's device,
 // one kernel copies all of them (and writes the records of `rec`); what it
-// must not touch (memory of another device or host, or not known to the
-// runtime, or not aligned to 4 bytes) goes by cudaMemcpyAsync, which takes
-// any address.  A field without source or destination is left out.
+// must not touch (copied_by_kernel()) goes by cudaMemcpyAsync.  A field without
+// source or destination is left out.
 struct Field
 {
     void* dst;
@@ -452,15 +452,17 @@ struct Field
 constexpr int kHostToDevice = 0, kDeviceToHost = 1, kOnDevice = 2;
 
 bool
-on_device(const aqua_ctx* x, const void* p)
+by_kernel(const aqua_ctx* x, const void* p)
 {
+    int current = -1;
     cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    if (cudaGetDevice(&current) != cudaSuccess ||
+        cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return at.type == cudaMemoryTypeDevice && at.device == x->device &&
-           (reinterpret_cast<uintptr_t>(p) & 3) == 0;
+    return copied_by_kernel(at.type == cudaMemoryTypeDevice, at.device, x->device,
+                            current, p);
 }
 
 aqua_status
@@ -474,7 +476,7 @@ copy_fields(aqua_ctx* x, const Field* f, size_t n, int kind,
             continue;
         // one end of each field is the context's own
         const void* user = rec.cid ? f[k].src : f[k].dst;
-        if (kind == kOnDevice && sp.n < kMaxSpans && on_device(x, user)) {
+        if (kind == kOnDevice && sp.n < kMaxSpans && by_kernel(x, user)) {
             sp.dst[sp.n] = static_cast<uint32_t*>(f[k].dst);
             sp.src[sp.n] = static_cast<const uint32_t*>(f[k].src);
             sp.words[sp.n++] = f[k].bytes / 4;

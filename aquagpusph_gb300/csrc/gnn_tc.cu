@@ -697,6 +697,7 @@ k_edge_mlp_tc(uint32_t E, const uint16_t* __restrict__ X, uint32_t ldx,
             load_idx(tile + stride);
             asm volatile("cp.async.wait_all;\n" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();  // every lane's copies, before lane 0's MMAs read them
             // the accumulator of the tile before has been read
             bool ok = n == 0;
             for (uint32_t it = 0; it < kWaitLimit && !ok; it++) {

@@ -174,6 +174,21 @@ build_consts(const aqua_params* p, Consts& c)
     auto ordinary = [](float x) { return x >= 0x1p-40f && x <= 0x1p120f; };
     c.quad_ok = ordinary(c.H) && c.H <= 0x1p40f && c.CONW > 0.f && c.CONF > 0.f &&
                 c.CONW <= 0x1p120f && c.CONF <= 0x1p120f;
+    // The quotients of a pair are exact while their numerators stay above
+    // 2^-102 (2^-47 of one must be a float); the smallest are W(q) CONW m and
+    // F(q) CONF m, with (2 - q)^4 and (2 - q)^3 in them.  On a lattice whose
+    // spacing divides the support six neighbours lie at its edge, at the
+    // smallest |2 - q| there is, 2^-23: masses from 2^-6 / CONW on cover that
+    // (with those pairs in the general expressions a 5.88M step at rest took 22.5
+    // ms, without 20.0).  Where masses may be smaller (by the density, for
+    // up to four spacings in h), fewer pairs at the edge are covered instead.
+    float least = p->n_sets ? p->refd[0] : 0.f;
+    for (uint32_t k = 1; k < p->n_sets; k++)
+        least = p->refd[k] < least ? p->refd[k] : least;
+    const bool heavy = least >= 1.f && c.CONF >= 0x1p-7f * c.CONW;
+    c.quad_mw = heavy ? 0x1p-6f : 0x1p-20f;
+    c.quad_mf = heavy ? 0x1p-13f : 0x1p-20f;
+    c.quad_aq = heavy ? -INFINITY : 0x1p-16f;
     return AQUA_OK;
 }
 

@@ -56,6 +56,9 @@ struct Consts
     float f_conf;       // F factor * CONF
     float f_over_w;     // f_conf / w_conw (clustered sweep)
     uint32_t quad_ok;   // H, CONW and CONF are in the range of quad_div
+    // smallest CONW m, CONF m and 2 - q of the pairs whose kernel factors
+    // quad_div takes
+    float quad_mw, quad_mf, quad_aq;
     // test-only: a bounded wait that completed is reported as timed out
     // (AQUA_ERR_TIMEOUT), so the error path runs with nothing in flight
     uint32_t debug_fake_timeout;

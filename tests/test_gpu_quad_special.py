@@ -42,3 +42,26 @@ def test_values_that_are_not_finite(dims, n, spread, name, value):
     else:
         a[n // 2] = value
     assert_same(c)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("scale", [1.0, 1e-3, 1e-6])
+@pytest.mark.parametrize("seed", range(4))
+def test_pairs_at_the_edge_of_the_support(dims, scale, seed):
+    """Neighbours within a few units in the last place of the support, inside,
+    on and outside it, and on a lattice whose spacing divides it: the smallest
+    kernel factors that there are, in and out of the range of the branch-free
+    quotients (by the masses)."""
+    n = 200
+    c = cloud(dims, n, 0.9, 17 + seed, 8, scale)
+    rng = np.random.default_rng(seed)
+    reach = np.float64(c.params.SUPPORT * c.params.H)
+    d = rng.normal(size=(n, dims))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    d[:2 * dims] = np.concatenate([np.eye(dims), -np.eye(dims)])
+    r = d * reach * (1.0 + rng.integers(-24, 25, (n, 1)) * 2.0 ** -24)
+    r[0] = 0.0
+    g = np.stack(np.meshgrid(*[np.arange(-2, 3)] * dims, indexing="ij"), -1).reshape(-1, dims)
+    r[1:1 + len(g)] = g[:n - 1] * reach / 4
+    c.r[:n, :dims] = r
+    assert_same(c)

@@ -1192,11 +1192,11 @@ aqua_launches_per_step(aqua_ctx* x)
     if (!x)
         return 0;
     // link-list (one launch, or begin, minmax, ncells, icell+hist and the
-    // radix passes), gather, clusters or chunks, [BI walls,] sweep, finalize
-    // [, motion]
+    // radix passes), gather, [octants,] clusters or chunks, [BI walls,] sweep
+    // [, by octant], finalize [, motion]
     return (small_linklist(x) ? 1u : 4u + x->passes) + 4u +
            (x->consts.boundary == AQUA_BOUNDARY_BI ? 1u : 0u) +
-           (x->has_motion ? 1u : 0u);
+           (sweep_clustered(x) && x->N > kOctantMin ? 2u : 0u) + (x->has_motion ? 1u : 0u);
 }
 
 }  // extern "C"

@@ -119,7 +119,9 @@ struct DevScalars
     uint32_t n_chunks;    // cell-aligned sweep chunks of this step
     uint32_t chunk_next;  // next chunk to hand out (work counter)
     uint32_t total_cells; // cells of all cases
-    uint32_t pad[4];
+    uint32_t by_octant;   // clusters of the sampled cells by whole octants
+    uint32_t by_cut;      // and as cuts of the curve (0: not sampled)
+    uint32_t pad[2];
 };
 
 // One set of the per-particle Variables (reference layout)

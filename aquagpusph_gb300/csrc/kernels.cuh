@@ -24,6 +24,11 @@ constexpr int kSweepClustered = 15;
 constexpr int kSweepVariants = 18;
 constexpr int kSweepClusteredDefault = 16;
 constexpr unsigned kSweepClusteredBlocks = 3;
+// Steps of more particles than this look whether the particles lie on a lattice
+// (k_octants) and are then swept by octant.  A step on a lattice with h = 2
+// spacings, by octant and by box: 316,544 particles 433 and 413 us, 5.88M 5.76
+// and 6.27 ms; the look and the kernel that returns at once cost 5 us.
+constexpr uint32_t kOctantMin = 600000;
 // Wendland C2 (Wendland{2D,3D}.hcl:44-66): the constant factors of W and F;
 // float products folded at compile time, as the OpenCL compiler folds them
 template<int D>
@@ -151,6 +156,15 @@ struct StepArgs
                        // the clustered sweep instead of posq/velq/pmq
     uint32_t cluster;  // particles per cluster of the quad sweep (4 or 8)
 };
+// Whether the clustered sweep of this step goes by octant: on a lattice the
+// sampled cells make at most 1.06 times the clusters (1.89M particles, h = 1.6
+// spacings: 2.18 ms, by box 2.60), sheared by less than a spacing 1.18 times and
+// more (5.88M, h = 2: 1.67 times; by octant 8.83, by box 7.87)
+__device__ __forceinline__ bool
+sweep_by_octant(const DevScalars* sc)
+{
+    return sc->by_cut > 0 && sc->by_octant * 8u <= sc->by_cut * 9u;
+}
 // gather / sweep of the step in the exact (IEEE, no FMA) or fast
 // (-use_fast_math) compilation
 template<int D>

@@ -105,6 +105,8 @@ k_begin(DevScalars* sc, CaseScalars* cs, uint32_t n_cases, uint2* cells,
     if (tid == 0) {
         sc->n_chunks = 0;
         sc->chunk_next = 0;
+        sc->by_octant = 0;
+        sc->by_cut = 0;
     }
     if (sc->err)
         return;
@@ -695,6 +697,8 @@ k_small_linklist(Consts c, const float* r, const int32_t* imove,
     if (b == 0 && t == 0) {
         sc->n_chunks = 0;
         sc->chunk_next = 0;
+        sc->by_octant = 0;
+        sc->by_cut = 0;
     }
     // an error of an earlier step: the blocks read it before any of this
     // launch's blocks can set it (rank 0, after the second cluster barrier)

@@ -92,6 +92,8 @@ __constant__ uint8_t kHilbert2[64] = {
 // (mixed with the elements the fluid's clusters lose their compact boxes: a
 // 5.88M step on a lattice took 6.73 ms, then 6.52, and a 5.9M call off it 8.57,
 // then 8.45), and crow holds the cell's neighbourhood as 9 rows of 3 cells.
+// Where the step is swept by octant (sweep_by_octant()), a cell's clusters are
+// octants (8 consecutive places), joined while they fit into 8, if all of them do.
 constexpr int kClusterThreads = 256;
 template<int D, bool CELLS>
 __global__ void __launch_bounds__(kClusterThreads)
@@ -104,8 +106,14 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
     __shared__ uint32_t s_cnt[NWARP][kNone];
     __shared__ uint2 s_warp[NWARP];
     __shared__ uint32_t s_base;
+    // the curve (constant memory serves one address at a time: 216 us for 5.88M
+    // particles, now 150)
+    __shared__ uint8_t s_place[64];
     if (__syncthreads_or(threadIdx.x == 0 && a.sc->err))
         return;  // one read for the whole block
+    const bool octants = CELLS && sweep_by_octant(a.sc);
+    if (threadIdx.x < 64)
+        s_place[threadIdx.x] = D == 3 ? kHilbert3[threadIdx.x] : kHilbert2[threadIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t s0 = blockIdx.x * kClusterThreads + threadIdx.x;
@@ -167,6 +175,9 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
             }
         }
         uint32_t walls = 0, probes = 0;
+        // clusters by octant: their number (0: none) and, lane k, the first
+        // place and the particles of cluster k
+        uint32_t nko = 0, oat = 0, on = 0;
         if (cnt > P || CELLS) {
             const float scale = (D == 3 ? 4.f : 8.f) * c.idist;
             auto place = [&](uint32_t s) -> uint32_t {
@@ -177,9 +188,9 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
                 const uint32_t x = (uint32_t)((p.x - cs.r_min[0]) * scale);
                 const uint32_t y = (uint32_t)((p.y - cs.r_min[1]) * scale);
                 if (D == 2)
-                    return kHilbert2[(x & 7u) | ((y & 7u) << 3)];
+                    return s_place[(x & 7u) | ((y & 7u) << 3)];
                 const uint32_t z = (uint32_t)((p.z - cs.r_min[2]) * scale);
-                return kHilbert3[(x & 3u) | ((y & 3u) << 2) | ((z & 3u) << 4)];
+                return s_place[(x & 3u) | ((y & 3u) << 2) | ((z & 3u) << 4)];
             };
             __syncwarp();
             s_cnt[warp][lane] = 0;
@@ -204,6 +215,29 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
                 const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= o)
                     x += y;
+            }
+            if (octants) {
+                uint32_t prev = 0, start = 0, open = 0;
+                bool fit = true;
+                for (int o = 0; o < 8; o++) {
+                    const uint32_t end = __shfl_sync(0xffffffffu, x, 4 * o + 3);
+                    const uint32_t co = end - prev;
+                    fit = fit && co <= 8u;
+                    if (open + co > 8u) {
+                        nko++;
+                        start = prev;
+                        open = 0;
+                    }
+                    open += co;
+                    prev = end;
+                    if (lane == (int)nko) {
+                        oat = start;
+                        on = open;
+                    }
+                }
+                nko++;
+                if (!fit || prev == 0)
+                    nko = 0;
             }
             __syncwarp();
             s_cnt[warp][2 * lane] = x - c0 - c1;
@@ -232,7 +266,8 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
         // at most as many as particles
         // (CELLS = false: only the order, the list has ceil(cnt / P) places)
         const uint32_t n0 = CELLS ? cnt - probes - walls : cnt, n1 = CELLS ? cnt - probes : cnt;
-        const uint32_t k0 = (n0 + P - 1u) / P, k1 = k0 + (n1 - n0 + P - 1u) / P;
+        const uint32_t k0 = nko ? nko : (n0 + P - 1u) / P;
+        const uint32_t k1 = k0 + (n1 - n0 + P - 1u) / P;
         const uint32_t nk = k1 + (cnt - n1 + P - 1u) / P;
         const uint32_t slot0 = CELLS ? first : base + cell.z;
         for (uint32_t k = lane; k < nk; k += 32) {
@@ -240,7 +275,8 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
                                 : k < k1 ? n0 + P * (k - k0)
                                          : n1 + P * (k - k1);
             const uint32_t end = k < k0 ? n0 : k < k1 ? n1 : cnt;
-            a.b.clu[slot0 + k] = make_uint2(first + at, min(P, end - at));
+            a.b.clu[slot0 + k] = k < nko ? make_uint2(first + oat, on)
+                                         : make_uint2(first + at, min(P, end - at));
         }
         if (CELLS) {
             if (lane == 0) {
@@ -259,6 +295,67 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
                     hi > lo ? make_uint2(lo, hi - lo) : make_uint2(0u, 0u);
             }
         }
+    }
+}
+
+// Looks whether the particles lie on a lattice: the cells of kOctantCells of them,
+// the clusters that the fluid makes by whole octants (joined while they fit into
+// 8; an octant of more counts as many as its particles) and as cuts of 8.
+constexpr uint32_t kOctantCells = 2048;
+__global__ void __launch_bounds__(256)
+k_octants(Consts c, StepArgs a)
+{
+    __shared__ uint32_t s_sum[2];
+    if (threadIdx.x < 2)
+        s_sum[threadIdx.x] = 0;
+    if (__syncthreads_or(threadIdx.x == 0 && a.sc->err))
+        return;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t w = blockIdx.x * 8u + (threadIdx.x >> 5);
+    const uint32_t s0 = (uint32_t)((uint64_t)w * a.N / kOctantCells);
+    const uint2 se = a.b.cells[a.skeys[s0]];
+    const CaseScalars& cs = a.cs[a.dst.cid[s0]];
+    const float scale = 4.f * c.idist;
+    uint32_t n = 0;  // lane o < 8: particles of octant o along the curve
+    for (uint32_t b = se.x; b < se.y; b += 32) {
+        uint32_t o = 8;
+        if (b + lane < se.y && a.dst.imove[b + lane] > 0) {
+            const float4 p = a.b.rec0[b + lane];
+            const uint32_t x = (uint32_t)((p.x - cs.r_min[0]) * scale) & 3u;
+            const uint32_t y = (uint32_t)((p.y - cs.r_min[1]) * scale) & 3u;
+            const uint32_t z = (uint32_t)((p.z - cs.r_min[2]) * scale) & 3u;
+            o = kHilbert3[x | (y << 2) | (z << 4)] / 8u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            const unsigned m = __ballot_sync(0xffffffffu, o == k);
+            if (lane == k)
+                n += (uint32_t)__popc(m);
+        }
+    }
+    uint32_t total = 0, clusters = 0, open = 0;
+    for (int o = 0; o < 8; o++) {
+        const uint32_t co = __shfl_sync(0xffffffffu, n, o);
+        total += co;
+        if (co > 8u) {
+            clusters += co;
+            continue;
+        }
+        if (open + co > 8u) {
+            clusters++;
+            open = 0;
+        }
+        open += co;
+    }
+    clusters += open > 0;
+    if (lane == 0 && total > 8u) {
+        atomicAdd(&s_sum[0], clusters);
+        atomicAdd(&s_sum[1], (total + 7u) / 8u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_sum[1]) {
+        atomicAdd(&a.sc->by_octant, s_sum[0]);
+        atomicAdd(&a.sc->by_cut, s_sum[1]);
     }
 }
 
@@ -488,6 +585,8 @@ launch_clusters(const Consts& c, const StepArgs& a, cudaStream_t s)
     if (a.N == 0)
         return cudaSuccess;
     const unsigned grid = (a.N + kClusterThreads - 1) / kClusterThreads;
+    if (D == 3 && a.clustered && a.N > kOctantMin)
+        k_octants<<<kOctantCells / 8, 256, 0, s>>>(c, a);
     if (D == 3 && a.clustered)
         k_cell_clusters<3, true><<<grid, kClusterThreads, 0, s>>>(c, a, a.b.rec0);
     else

@@ -23,17 +23,26 @@ launch_sweep_cl(const Consts& c, const StepArgs& a, unsigned grid,
 {
     if (a.N == 0)
         return cudaSuccess;
-    k_sweep_cl<kClWarps, kClRecords, 3>
-        <<<grid, kClWarps * 32, sizeof(ClSmem<kClWarps, kClRecords>), s>>>(c, a);
+    if (a.N > kOctantMin)
+        k_sweep_cl<kClWarps, kClRecords, 3, true>
+            <<<grid, kClWarps * 32, sizeof(ClSmem<kClWarps, kClRecords, true>), s>>>(c, a);
+    k_sweep_cl<kClWarps, kClRecords, 3, false>
+        <<<grid, kClWarps * 32, sizeof(ClSmem<kClWarps, kClRecords, false>), s>>>(c, a);
     return cudaGetLastError();
 }
 
 cudaError_t
 prepare_sweep_cl()
 {
-    return cudaFuncSetAttribute(k_sweep_cl<kClWarps, kClRecords, 3>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(ClSmem<kClWarps, kClRecords>));
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_sweep_cl<kClWarps, kClRecords, 3, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(ClSmem<kClWarps, kClRecords, true>));
+    return e != cudaSuccess
+               ? e
+               : cudaFuncSetAttribute(k_sweep_cl<kClWarps, kClRecords, 3, false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(ClSmem<kClWarps, kClRecords, false>));
 }
 
 }  // namespace fast

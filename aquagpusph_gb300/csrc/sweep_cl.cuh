@@ -33,11 +33,21 @@
 // lattice most cells hold 9 clusters, and seven warps would wait for the
 // ninth.
 //
-// Instruction issue bounds it (72% of the slots, 24 warps an SM by shared
-// memory).  Clusters by octant, with one mask per staged record for all eight,
-// were 5 to 7 of 8 full off the lattice: 5.9M sheared particles 9.39 ms a call,
-// now 8.2; 406,402: 1.09 ms, now 0.80.  On a lattice at rest octants are perfect
-// clusters, and those masks were 9% cheaper (5.88M: 5.75 ms a step, now 6.28).
+// Steps on a lattice (sweep_by_octant()) are swept by octant: clusters are whole
+// octants of the cell, and instead of a box test per record and cluster the block
+// classifies every staged record once into a 16-bit mask, the octant boxes that
+// it comes within the support of (a box per octant, spanning, per axis and half,
+// the cell's particles there), in the low byte for a fluid record and the high
+// byte for a boundary element.  Each cluster's scan reads those masks, four
+// records per lane.
+//
+// Instruction issue bounds both (72% of the slots, 24 warps an SM by shared
+// memory).  Off the lattice octants fill their clusters 5 to 7 of 8: 5.9M sheared
+// particles 9.39 ms a call, by box 8.2; 406,402: 1.09 ms, by box 0.79.  On a
+// lattice at rest octants are perfect clusters and finding their neighbours takes
+// 1,365 instructions of a warp per cluster in place of 2,060: 5.88M particles 5.76
+// ms a step, by box 6.27.  Both in one kernel, chosen by cell, were 7 to 15% slower
+// in all cases (registers, instruction cache, shared memory).
 //
 // Boundary elements reach fluid particles through a second list (the BIe
 // wall sums), which also serves the elastic bounce and PST of the
@@ -63,17 +73,34 @@ constexpr int kClMaxPieces = 32;     // staged runs per pass
 constexpr uint32_t kClWaitLimit = 1u << 22;
 constexpr uint32_t kClShare = 8;     // warps that share a cell's last clusters
 constexpr int kClSums = 13;          // sums of a particle
+// by octant: bit o (o < 8) of a fluid record, bit 8 + o of a boundary element =
+// within the support of the cell's octant box o
+constexpr uint32_t kMaskWallShift = 8;
+
+// Shared memory of the kind of sweep: the sums of a shared cluster, by part, or
+template<int CAP, bool OCT>
+struct ClKind
+{
+    float part[kClShare][kClSums][8];
+};
+// (by octant) per staged record its octants by kind, and the octants' boxes
+template<int CAP>
+struct ClKind<CAP, true>
+{
+    alignas(8) uint16_t mask[CAP + 4];
+    float ivl[12];               // axis a, half h: [lo, hi] at 4 a + 2 h
+};
 
 // Shared memory of one block: staged records (CAP + 1: the last is a zero
 // record that pads the lists to whole quads), per-warp lists, staged runs
-template<int NW, int CAP>
+template<int NW, int CAP, bool OCT>
 struct ClSmem
 {
     float4 r0[CAP + 1];
     float4 r1[CAP + 1];
     uint16_t list[NW][kClListCap + 4];   // + room for the padding quad
     uint16_t wall[NW][kClWallCap + 4];
-    float part[kClShare][kClSums][8];    // sums of a shared cluster, by part
+    ClKind<CAP, OCT> kind;
     uint32_t wn[NW];                     // entries of wall[]; bit 31: overflowed
     uint4 piece[kClMaxPieces];   // (slot, sorted first, count, -)
     uint2 row[9];                // (sorted first, count) of each row
@@ -84,6 +111,17 @@ struct ClSmem
     uint64_t mbar;
 };
 
+// Octant (0-7, x fastest) of a position inside its cell: the halves of the
+// cell along each axis (cells are (support h) wide from the case's r_min)
+__device__ __forceinline__ uint32_t
+cl_octant(const float4 p, const CaseScalars& cs, float sc2)
+{
+    const uint32_t ox = (uint32_t)((p.x - cs.r_min[0]) * sc2) & 1u;
+    const uint32_t oy = (uint32_t)((p.y - cs.r_min[1]) * sc2) & 1u;
+    const uint32_t oz = (uint32_t)((p.z - cs.r_min[2]) * sc2) & 1u;
+    return ox | (oy << 1) | (oz << 2);
+}
+
 // Everything after the sums for sorted particle i of a cluster (the same
 // steps and expressions as the epilogue of k_sweep): Shepard, the BIe and
 // cfd rates, delta-SPH, elastic bounce, midpoint relax and corrector, PST,
@@ -93,14 +131,14 @@ struct ClSmem
 // PST come from the cluster's staged wall lists (those of warps l0 .. l0 + L
 // - 1, in order) or, when `walls_global`, from the per-cell index ranges of
 // the 27 cells around `key` in global memory.
-template<int NW, int CAP>
+template<typename Smem>
 __device__ __forceinline__ float
 sweep_cl_finish(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
                 int im, bool want, bool fluid, bool sensor, bool store,
                 float dt, const float4 r0i, const float4 r1i, float shep,
                 float gp0, float gp1, float gp2, float lu0, float lu1,
                 float lu2, float du, float lp, float gw0, float gw1, float gw2,
-                float dbi, bool walls_global, const ClSmem<NW, CAP>& S,
+                float dbi, bool walls_global, const Smem& S,
                 uint32_t l0, uint32_t L, uint32_t key, const CaseScalars& cas)
 {
     if (!valid)
@@ -328,14 +366,16 @@ cl_wait(uint64_t* mbar, uint32_t parity)
     return done != 0;
 }
 
-// The persistent clustered sweep.  NW warps per block, CAP staged records
-// per pass.
-template<int NW, int CAP, int MINB>
+// The persistent clustered sweep.  NW warps per block, CAP staged records per
+// pass; OCT: by octant, the steps that k_octants chose it for.
+template<int NW, int CAP, int MINB, bool OCT>
 __global__ void __launch_bounds__(NW * 32, MINB)
 k_sweep_cl(Consts c, StepArgs a)
 {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    ClSmem<NW, CAP>& S = *reinterpret_cast<ClSmem<NW, CAP>*>(smem_raw);
+    if (sweep_by_octant(a.sc) != OCT)
+        return;  // the same for every block
+    ClSmem<NW, CAP, OCT>& S = *reinterpret_cast<ClSmem<NW, CAP, OCT>*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int q = lane >> 3;         // neighbour slot (lanes 8 q .. 8 q + 7)
     const int mq = lane & 7;         // particle of the cluster
@@ -408,16 +448,59 @@ k_sweep_cl(Consts c, StepArgs a)
         parity ^= 1u;
         // zero records up to the next multiple of 64, so that the scan tests
         // no bounds
-        const uint32_t n = min(S.total - p * (uint32_t)CAP, (uint32_t)CAP);
-        if (n + tid < ((n + 63u) & ~63u))
-            S.r0[n + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        if constexpr (!OCT) {
+            const uint32_t n = min(S.total - p * (uint32_t)CAP, (uint32_t)CAP);
+            if (n + tid < ((n + 63u) & ~63u))
+                S.r0[n + tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        }
         __syncthreads();  // S.piece / S.nstaged visible; the vote below
         const bool bad = __syncthreads_or(!ok);
         if (bad) {
             if (tid == 0)
                 atomicOr(&a.sc->err, kErrTimeout);
             return false;
+        }
+        if constexpr (OCT) {
+            // classify the staged records once for all the cell's clusters:
+            // their kind, and which octant boxes of the cell (S.ivl) they come
+            // within the support of (box distance per axis and half, summed
+            // over the 8 combinations)
+            {
+                const uint32_t nst = S.nstaged;
+                float lo[6], hi[6];
+#pragma unroll
+                for (int q = 0; q < 6; q++) {
+                    lo[q] = S.kind.ivl[2 * q];
+                    hi[q] = S.kind.ivl[2 * q + 1];
+                }
+                for (uint32_t k = tid; k < nst; k += NW * 32) {
+                    const float4 pc = S.r0[k];
+                    uint32_t m = 0u;
+                    if (pc.w != 0.f) {
+                        const float x[3] = { pc.x, pc.y, pc.z };
+                        float d2[6];
+#pragma unroll
+                        for (int q = 0; q < 6; q++) {
+                            const float d = fmaxf(fmaxf(lo[q] - x[q >> 1], x[q >> 1] - hi[q]), 0.f);
+                            d2[q] = d * d;
+                        }
+                        // (x half, y half) combinations, then z
+                        const float dxy[4] = { d2[0] + d2[2], d2[1] + d2[2],
+                                               d2[0] + d2[3], d2[1] + d2[3] };
+#pragma unroll
+                        for (int o = 0; o < 8; o++)
+                            if (dxy[o & 3] + d2[4 + (o >> 2)] < R2)
+                                m |= 1u << o;
+                        if (pc.w < 0.f)
+                            m <<= kMaskWallShift;
+                    }
+                    S.kind.mask[k] = (uint16_t)m;
+                }
+                if (tid < 3)
+                    S.kind.mask[nst + tid] = 0;  // read with the last records' group of 4
+            }
+            __syncthreads();
         }
         return true;
     };
@@ -475,6 +558,56 @@ k_sweep_cl(Consts c, StepArgs a)
         __syncthreads();
         const uint32_t npass = (S.total + CAP - 1) / CAP;
         const bool single = npass <= 1;
+        if constexpr (OCT) {
+            if (warp == NW - 1) {
+                // the octant boxes of the cell: per axis and half, the extent of
+                // the cell's particles that take neighbour sums (probes apart);
+                // an empty half stays [+inf, -inf] and is never within reach.
+                // Ready before the classification (stage's barrier).
+                const float sc2 = 2.f * c.idist;
+                float bl[6], bh[6];
+#pragma unroll
+                for (int q = 0; q < 6; q++) {
+                    bl[q] = INFINITY;
+                    bh[q] = -INFINITY;
+                }
+                for (uint32_t sidx = wc.x + lane; sidx < wc.y; sidx += 32) {
+                    const int imv = T.imove[sidx];
+                    if (imv < -3 || imv > 1 || imv == 0)
+                        continue;
+                    const float4 p = a.b.rec0[sidx];
+                    const uint32_t o = cl_octant(p, cas, sc2);
+                    const float x[3] = { p.x, p.y, p.z };
+#pragma unroll
+                    for (int ax = 0; ax < 3; ax++) {
+                        // constant indices (registers): half 0 or 1 by select
+                        const bool up = (o >> ax) & 1u;
+                        bl[2 * ax] = up ? bl[2 * ax] : fminf(bl[2 * ax], x[ax]);
+                        bh[2 * ax] = up ? bh[2 * ax] : fmaxf(bh[2 * ax], x[ax]);
+                        bl[2 * ax + 1] = up ? fminf(bl[2 * ax + 1], x[ax]) : bl[2 * ax + 1];
+                        bh[2 * ax + 1] = up ? fmaxf(bh[2 * ax + 1], x[ax]) : bh[2 * ax + 1];
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 6; q++) {
+                    for (int o = 16; o > 0; o >>= 1) {
+                        bl[q] = fminf(bl[q], __shfl_xor_sync(0xffffffffu, bl[q], o));
+                        bh[q] = fmaxf(bh[q], __shfl_xor_sync(0xffffffffu, bh[q], o));
+                    }
+                }
+                if (lane < 6) {
+                    float l = bl[0], h = bh[0];
+#pragma unroll
+                    for (int q = 1; q < 6; q++)
+                        if (lane == (uint32_t)q) {
+                            l = bl[q];
+                            h = bh[q];
+                        }
+                    S.kind.ivl[2 * lane] = l;
+                    S.kind.ivl[2 * lane + 1] = h;
+                }
+            }
+        }
         bool failed = !stage(0);
         if (tid == 0)
             w_next = fetch();  // consumed at the end of this cell
@@ -483,7 +616,8 @@ k_sweep_cl(Consts c, StepArgs a)
         // finished by the first warps.  Several passes: waves of NW whole
         // clusters, each wave re-staging every pass.
         const uint32_t rest = n_cl % kClShare;
-        const uint32_t share = single && rest && NW == (int)kClShare ? kClShare / rest : 1u;
+        const uint32_t share =
+            !OCT && single && rest && NW == (int)kClShare ? kClShare / rest : 1u;
         const uint32_t whole = share > 1u ? n_cl - rest : n_cl;
         const uint32_t parts = share > 1u ? rest * share : 0u;
         bool combine = false;
@@ -585,9 +719,16 @@ k_sweep_cl(Consts c, StepArgs a)
                     }
                 };
 
-                // the box of the cluster's particles that take sums
+                // the box of the cluster's particles that take sums, or the
+                // octants they lie in (each box holds its particles, so the
+                // candidates within the support of any of these are all)
                 float lo[3], hi[3];
-                {
+                uint32_t omask = 0;
+                if constexpr (OCT) {
+                    omask = __reduce_or_sync(
+                        0xffffffffu,
+                        want && !sensor ? 1u << cl_octant(r0i, cas, 2.f * c.idist) : 0u);
+                } else {
                     const float x[3] = { r0i.x, r0i.y, r0i.z };
 #pragma unroll
                     for (int d = 0; d < 3; d++) {
@@ -661,71 +802,130 @@ k_sweep_cl(Consts c, StepArgs a)
                     }
                     uint32_t fill = 0;
                     uint32_t wdone = wfill;  // wall entries already summed
-                    const uint32_t g = part ? u % share : 0u, G = part ? share : 1u;
-                    const uint32_t rounds = (nst + 63u) / 64u;
-                    const uint32_t k_end = rounds * (g + 1u) / G * 64u;
-                    // 64 records per round, two per lane, listed in staging
-                    // order
-                    for (uint32_t base = rounds * g / G * 64u; base < k_end; base += 64) {
-                        unsigned bf[2];
-                        bool fl[2], wa[2];
+                    // a full wall list: sum it, and let the epilogue walk the
+                    // walls from global memory
+                    auto wall_room = [&](uint32_t wtot) {
+                        if (wfill + wtot <= (uint32_t)kClWallCap)
+                            return;
+                        __syncwarp();
+                        const uint32_t n = wfill - wdone;
+                        if (lane < (int)((4 - (n & 3)) & 3))
+                            wl[wfill + lane] = (uint16_t)CAP;
+                        __syncwarp();
+                        drain(wl + wdone, (n + 3) / 4, true);
+                        __syncwarp();
+                        wfill = 0;
+                        wdone = 0;
+                        walls_global = true;
+                    };
+                    // the listed quads
+                    auto take = [&]() {
+                        __syncwarp();
+                        const uint32_t nq = fill / 4;
+                        drain(list, nq, false);
+                        __syncwarp();
+                        const uint32_t rem = fill - 4 * nq;
+                        uint16_t mv = 0;
+                        if ((uint32_t)lane < rem)
+                            mv = list[4 * nq + lane];
+                        __syncwarp();
+                        if ((uint32_t)lane < rem)
+                            list[lane] = mv;
+                        fill = rem;
+                    };
+                    if constexpr (OCT) {
+                        // the boundary elements matter to fluid particles only
+                        const uint32_t wmask = any_fluid ? omask << kMaskWallShift : 0u;
+                        // 128 records per round, four per lane (records 4l ..
+                        // 4l+3), listed in staging order
+                        for (uint32_t base = 0; base < nst; base += 128) {
+                            const uint32_t k0 = base + 4u * lane;
+                            uint2 mm = make_uint2(0u, 0u);
+                            if (k0 < nst)
+                                mm = *reinterpret_cast<const uint2*>(&S.kind.mask[k0]);
+                            const uint32_t m[4] = { mm.x & 0xffffu, mm.x >> 16, mm.y & 0xffffu, mm.y >> 16 };
+                            bool fl[4], wa[4];
+                            unsigned bw[4];
+                            uint32_t before = 0, wbefore = 0, tot = 0, wtot = 0;
 #pragma unroll
-                        for (int v = 0; v < 2; v++) {
-                            const float4 r = S.r0[base + 32u * v + lane];
-                            const float dx = fmaxf(fmaxf(lo[0] - r.x, r.x - hi[0]), 0.f);
-                            const float dy = fmaxf(fmaxf(lo[1] - r.y, r.y - hi[1]), 0.f);
-                            const float dz = fmaxf(fmaxf(lo[2] - r.z, r.z - hi[2]), 0.f);
-                            const bool in = dx * dx + dy * dy + dz * dz < R2;
-                            fl[v] = in && r.w > 0.f;
-                            // the boundary elements matter to fluid only
-                            wa[v] = in && r.w < 0.f && any_fluid;
-                            bf[v] = __ballot_sync(0xffffffffu, fl[v]);
-                        }
-                        if (fl[0])
-                            list[fill + (uint32_t)__popc(bf[0] & lt)] = (uint16_t)(base + lane);
-                        fill += (uint32_t)__popc(bf[0]);
-                        if (fl[1])
-                            list[fill + (uint32_t)__popc(bf[1] & lt)] = (uint16_t)(base + 32u + lane);
-                        fill += (uint32_t)__popc(bf[1]);
-                        if (__any_sync(0xffffffffu, wa[0] || wa[1])) {
-                            const unsigned bw[2] = { __ballot_sync(0xffffffffu, wa[0]),
-                                                     __ballot_sync(0xffffffffu, wa[1]) };
-                            const uint32_t wtot = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1]);
-                            if (wfill + wtot > (uint32_t)kClWallCap) {
-                                // the wall list is full: sum it, and let the
-                                // epilogue walk the walls from global memory
-                                __syncwarp();
-                                const uint32_t n = wfill - wdone;
-                                if (lane < (int)((4 - (n & 3)) & 3))
-                                    wl[wfill + lane] = (uint16_t)CAP;
-                                __syncwarp();
-                                drain(wl + wdone, (n + 3) / 4, true);
-                                __syncwarp();
-                                wfill = 0;
-                                wdone = 0;
-                                walls_global = true;
+                            for (int u = 0; u < 4; u++) {
+                                fl[u] = (m[u] & omask) != 0u;
+                                wa[u] = (m[u] & wmask) != 0u;
+                                const unsigned bf = __ballot_sync(0xffffffffu, fl[u]);
+                                bw[u] = __ballot_sync(0xffffffffu, wa[u]);
+                                before += (uint32_t)__popc(bf & lt);
+                                tot += (uint32_t)__popc(bf);
+                                wtot |= bw[u];
                             }
-                            uint32_t wbefore = (uint32_t)__popc(bw[0] & lt);
-                            if (wa[0])
-                                wl[wfill + wbefore] = (uint16_t)(base + lane);
-                            wbefore = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1] & lt);
-                            if (wa[1])
-                                wl[wfill + wbefore] = (uint16_t)(base + 32u + lane);
-                            wfill += wtot;
+                            {
+                                uint32_t p = fill + before;
+#pragma unroll
+                                for (int u = 0; u < 4; u++)
+                                    if (fl[u])
+                                        list[p++] = (uint16_t)(k0 + u);
+                            }
+                            fill += tot;
+                            if (wtot) {
+#pragma unroll
+                                for (int u = 0; u < 4; u++)
+                                    wbefore += (uint32_t)__popc(bw[u] & lt);
+                                wtot = 0;
+#pragma unroll
+                                for (int u = 0; u < 4; u++)
+                                    wtot += (uint32_t)__popc(bw[u]);
+                                wall_room(wtot);
+                                uint32_t q = wfill + wbefore;
+#pragma unroll
+                                for (int u = 0; u < 4; u++)
+                                    if (wa[u])
+                                        wl[q++] = (uint16_t)(k0 + u);
+                                wfill += wtot;
+                            }
+                            if (fill > (uint32_t)(kClListCap - 128))
+                                take();
                         }
-                        if (fill > (uint32_t)(kClListCap - 64)) {
-                            __syncwarp();
-                            const uint32_t nq = fill / 4;
-                            drain(list, nq, false);
-                            __syncwarp();
-                            const uint32_t rem = fill - 4 * nq;
-                            uint16_t mv = 0;
-                            if ((uint32_t)lane < rem)
-                                mv = list[4 * nq + lane];
-                            __syncwarp();
-                            if ((uint32_t)lane < rem)
-                                list[lane] = mv;
-                            fill = rem;
+                    } else {
+                        const uint32_t g = part ? u % share : 0u, G = part ? share : 1u;
+                        const uint32_t rounds = (nst + 63u) / 64u;
+                        const uint32_t k_end = rounds * (g + 1u) / G * 64u;
+                        // 64 records per round, two per lane, listed in staging
+                        // order
+                        for (uint32_t base = rounds * g / G * 64u; base < k_end; base += 64) {
+                            unsigned bf[2];
+                            bool fl[2], wa[2];
+#pragma unroll
+                            for (int v = 0; v < 2; v++) {
+                                const float4 r = S.r0[base + 32u * v + lane];
+                                const float dx = fmaxf(fmaxf(lo[0] - r.x, r.x - hi[0]), 0.f);
+                                const float dy = fmaxf(fmaxf(lo[1] - r.y, r.y - hi[1]), 0.f);
+                                const float dz = fmaxf(fmaxf(lo[2] - r.z, r.z - hi[2]), 0.f);
+                                const bool in = dx * dx + dy * dy + dz * dz < R2;
+                                fl[v] = in && r.w > 0.f;
+                                // the boundary elements matter to fluid only
+                                wa[v] = in && r.w < 0.f && any_fluid;
+                                bf[v] = __ballot_sync(0xffffffffu, fl[v]);
+                            }
+                            if (fl[0])
+                                list[fill + (uint32_t)__popc(bf[0] & lt)] = (uint16_t)(base + lane);
+                            fill += (uint32_t)__popc(bf[0]);
+                            if (fl[1])
+                                list[fill + (uint32_t)__popc(bf[1] & lt)] = (uint16_t)(base + 32u + lane);
+                            fill += (uint32_t)__popc(bf[1]);
+                            if (__any_sync(0xffffffffu, wa[0] || wa[1])) {
+                                const unsigned bw[2] = { __ballot_sync(0xffffffffu, wa[0]),
+                                                         __ballot_sync(0xffffffffu, wa[1]) };
+                                const uint32_t wtot = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1]);
+                                wall_room(wtot);
+                                uint32_t wbefore = (uint32_t)__popc(bw[0] & lt);
+                                if (wa[0])
+                                    wl[wfill + wbefore] = (uint16_t)(base + lane);
+                                wbefore = (uint32_t)__popc(bw[0]) + (uint32_t)__popc(bw[1] & lt);
+                                if (wa[1])
+                                    wl[wfill + wbefore] = (uint16_t)(base + 32u + lane);
+                                wfill += wtot;
+                            }
+                            if (fill > (uint32_t)(kClListCap - 64))
+                                take();
                         }
                     }
                     // the rest of both lists, padded with the zero record
@@ -747,17 +947,19 @@ k_sweep_cl(Consts c, StepArgs a)
                 // ---- the four partial sums of each particle
                 float* acc[kClSums] = { &shep, &gp0, &gp1, &gp2, &lu0, &lu1, &lu2,
                                         &du, &lp, &gw0, &gw1, &gw2, &dbi };
-                if (combine) {
+                if (!OCT && combine) {
                     // the parts of the cluster, in order
                     walls_global = false;
                     for (uint32_t k = 0; k < share; k++)
                         walls_global = walls_global || (S.wn[warp * share + k] >> 31);
+                    if constexpr (!OCT) {
 #pragma unroll
-                    for (int k = 0; k < kClSums; k++) {
-                        float v = S.part[warp * share][k][mq];
-                        for (uint32_t g = 1; g < share; g++)
-                            v = v + S.part[warp * share + g][k][mq];
-                        *acc[k] = v;
+                        for (int k = 0; k < kClSums; k++) {
+                            float v = S.kind.part[warp * share][k][mq];
+                            for (uint32_t g = 1; g < share; g++)
+                                v = v + S.kind.part[warp * share + g][k][mq];
+                            *acc[k] = v;
+                        }
                     }
                 } else {
 #pragma unroll
@@ -770,15 +972,16 @@ k_sweep_cl(Consts c, StepArgs a)
                     if (lane == 0)
                         S.wn[warp] = wfill | (part && walls_global ? 0x80000000u : 0u);
                 }
-                if (part) {
-                    if (q == 0)
+                if (!OCT && part) {
+                    if constexpr (!OCT)
+                        if (q == 0)
 #pragma unroll
-                        for (int k = 0; k < kClSums; k++)
-                            S.part[u][k][mq] = *acc[k];
+                            for (int k = 0; k < kClSums; k++)
+                                S.kind.part[u][k][mq] = *acc[k];
                 } else if (have) {
                     __syncwarp();
                     shep = shep + shep;  // the pair sums hold half of it
-                    const float v = sweep_cl_finish<NW, CAP>(
+                    const float v = sweep_cl_finish(
                         c, a, i, valid, im, want, fluid, sensor, q == 0, dt,
                         r0i, r1i, shep, gp0, gp1, gp2, lu0, lu1, lu2, du, lp,
                         gw0, gw1, gw2, dbi, walls_global, S,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "aqua_internal.cuh"
+#include "arith.cuh"
 
 namespace aqua {
 

@@ -20,7 +20,8 @@ def lib(tmp_path_factory):
     subprocess.run([build.nvcc()] + build._flags("gnn_tc.cu") +
                    ["-shared", os.path.join(HERE, "arith_check.cu"), "-o", out], check=True)
     so = ctypes.CDLL(out)
-    for name in ("check_silu_grad",):
+    for name in ("check_silu_grad", "check_sqrt", "check_div", "check_div_product",
+                 "check_div_small"):
         getattr(so, name).restype = ctypes.c_longlong
     return so
 
@@ -33,3 +34,25 @@ def test_silu_gradient(lib):
     """Every float up to 128, both signs; infinity and NaN."""
     assert lib.check_silu_grad(0, bits(128.0)) == 0
     assert lib.check_silu_grad(bits(np.inf), bits(np.nan)) == 0
+
+
+def test_quad_sqrt(lib):
+    """Every mantissa of two binades, zero, and every float at the ends of the range."""
+    assert lib.check_sqrt(bits(1.0), bits(4.0)) == 0
+    assert lib.check_sqrt(bits(2.0 ** -100), bits(2.0 ** -99)) == 0
+    assert lib.check_sqrt(bits(2.0 ** 99), bits(2.0 ** 100)) == 0
+    assert lib.check_sqrt(0, 0) == 0
+
+
+def test_quad_div(lib):
+    """Every mantissa of the divisor, with the numerators whose quotients lie
+    nearest to the middle between two floats."""
+    assert lib.check_div(64) == 0
+
+
+def test_quad_div_by_a_product_of_densities(lib):
+    assert lib.check_div_product(64) == 0
+
+
+def test_quad_div_of_the_smallest_numerators(lib):
+    assert lib.check_div_small() == 0

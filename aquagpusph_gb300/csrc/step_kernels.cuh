@@ -22,8 +22,8 @@
 //
 // With the improved Euler scheme (basic/time_scheme/improved_euler.xml, BI
 // walls) k_gather runs the improved_euler.cl predictor in place of the
-// midpoint backups, copies and advance, and the sweep epilogue its corrector
-// in place of the midpoint relax and corrector.
+// midpoint backups, copies and advance, and the quad sweep (sweep_quad.cuh) its
+// corrector in place of the midpoint relax and corrector.
 //
 // Every accumulator visits its neighbours in the reference order (27 cells,
 // x offset outermost; particles of a cell in sorted order) and each
@@ -447,7 +447,7 @@ k_gather(Consts c, StepArgs a)
 // neighbour cells of the warp's cell.  The scan checks the queues every 32
 // candidates, where they have room for at least 32 more, so a queue never
 // overflows.
-template<int D, int NT, int NQ, typename QE, bool BULK, bool BI, int MODE>
+template<int D, int NT, int NQ, typename QE, bool BULK, int MODE>
 __device__ __forceinline__ float
 sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
                QE* queue, uint32_t* cstart, float4* grp2, uint64_t* mbar,
@@ -465,12 +465,8 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
     const uint32_t nxy = cas.n_cells[0] * cas.n_cells[1];
     const uint32_t key_i = a.skeys[i];
     const bool fluid = valid && (im == 1), sensor = valid && (im == 0);
-    // BIe: the Shepard sum runs for -3 <= imove <= 1 (cfd/Shepard.cl); BI:
-    // the walls are handled by k_bi_walls, fluid and probes take fluid
-    // neighbours only here and the walls in the epilogue
-    constexpr bool bie = !BI;  // the wall formulation is a compile-time choice
-    const bool want_shep = valid && (bie ? (im >= -3) && (im <= 1)
-                                         : (im == 0) || (im == 1));
+    // the Shepard sum runs for -3 <= imove <= 1 (cfd/Shepard.cl)
+    const bool want_shep = valid && (im >= -3) && (im <= 1);
 
     float shep = 0.f;
     float gp[3] = { 0.f, 0.f, 0.f }, lu[3] = { 0.f, 0.f, 0.f };
@@ -837,7 +833,7 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
                 float d0, d1, d2;
                 const float rr = sep(pj, d0, d1, d2);
                 const bool take = want_shep &&
-                                  (jm == 1 || (bie && fluid && jm == -3)) &&
+                                  (jm == 1 || (fluid && jm == -3)) &&
                                   rr < c.q2_reject;
                 if (take) {
                     if constexpr (kFastArith)
@@ -856,7 +852,7 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
                 rr = rr + d2 * d2;
             }
             const bool take = want_shep &&
-                              (jm == 1 || (bie && fluid && jm == -3)) &&
+                              (jm == 1 || (fluid && jm == -3)) &&
                               rr < c.q2_reject;
             if (take) {
                 if constexpr (sizeof(QE) == 2)
@@ -903,67 +899,6 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
             du = du * rho_i;
         }
     }
-    if constexpr (BI) {
-        // BI walls: the analytic Shepard factor (BI/Shepard.cl compute) of
-        // fluid particles and probes, and the wall terms of the fluid
-        // particles (BI/Interactions.cl) added onto the completed fluid
-        // sums, walls in visiting order
-        if (im == -3)
-            return c.dt_fixed;  // done by k_bi_walls
-        shep = 1.f;
-        bool self_added = false;
-        for (int k = 0; k < NC; k++) {
-            const uint32_t cn = neighbour_cell<D>(key_i, k, nx, nxy);
-            const uint2 se = a.b.wall_range[cn];  // empty: x > y
-            for (uint32_t j = se.x; j < se.y; j++) {
-                const float4 pj = a.b.posq[j];
-                if (__float_as_int(pj.w) != -3)
-                    continue;
-                float d[3];
-                d[0] = pj.x - ri[0];
-                d[1] = pj.y - ri[1];
-                d[2] = (D == 3) ? pj.z - ri[2] : 0.f;
-                const float q = sqrtf(dot_d<D>(d, d)) / c.H;
-                if (q >= c.SUPPORT)
-                    continue;
-                float nj[3], tj[3], bj[3];
-                load_normal<D>(a.dst.normal, j, nj);
-                load_normal<D>(a.dst.tangent, j, tj);
-                load_normal<D>(a.dst.binormal, j, bj);
-                const float area = a.b.pmq[j].y;
-                const float rn = dot_d<D>(d, nj);
-                if ((rn > -1e-8f * c.H) && (rn < 1e-8f * c.H)) {
-                    if (!self_added) {
-                        const float rt = fabsf(dot_d<D>(d, tj));
-                        const float rb = fabsf(dot_d<D>(d, bj));
-                        const float dr = 0.55f * powf(area, 1.f / (c.DIMS - 1.f));
-                        if ((rt <= dr) && (rb <= dr)) {
-                            self_added = true;
-                            shep = shep - 0.5f;
-                        }
-                    }
-                } else {
-                    const float rt = fabsf(dot_d<D>(d, tj));
-                    const float rb = fabsf(dot_d<D>(d, bj));
-                    shep = shep + (rn * c.CONW * kernel_sp<D>(q) * area +
-                                   kernel_sd<D>(fabsf(rn), rt, rb, area));
-                }
-                if (fluid) {
-                    const float pw = a.b.pmq[j].x;
-                    const float4 vw = a.b.velq[j];
-                    const float w = kernel_w<D>(q) * c.CONW * area;
-                    const float sg = (p_i + pw) / rho_i * w;
-                    for (int kk = 0; kk < D; kk++)
-                        gp[kk] = gp[kk] + sg * nj[kk];
-                    float dv[3];
-                    dv[0] = vw.x - uiv[0];
-                    dv[1] = vw.y - uiv[1];
-                    dv[2] = (D == 3) ? vw.z - uiv[2] : 0.f;
-                    du = du + rho_i * dot_d<D>(dv, nj) * w;
-                }
-            }
-        }
-    }
     if (a.b.shepard)
         a.b.shepard[i] = want_shep ? shep : 0.f;
 
@@ -972,7 +907,7 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
     float gpf[4] = { 0.f, 0.f, 0.f, 0.f }, luf[4] = { 0.f, 0.f, 0.f, 0.f };
     float gwf[4] = { 0.f, 0.f, 0.f, 0.f };
     float div_u = 0.f;
-    if (fluid && bie) {
+    if (fluid) {
         for (int k = 0; k < D; k++) {
             gpf[k] = gp[k];
             luf[k] = lu[k];
@@ -983,17 +918,6 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
         for (int k = 0; k < VS; k++)
             gpf[k] = gpf[k] + s2 * gwf[k];
         div_u = du - 2.f * rho_i * (dot_full<D>(ui_full, gwf) + dbi);
-    } else if (fluid) {
-        // BI/Shepard.cl apply: renormalise by the analytic Shepard factor
-        for (int k = 0; k < D; k++) {
-            gpf[k] = gp[k];
-            luf[k] = lu[k];
-        }
-        for (int k = 0; k < VS; k++) {
-            gpf[k] = gpf[k] / shep;
-            luf[k] = luf[k] / shep;
-        }
-        div_u = du / shep;
     }
     if (a.extras) {
         Vec<D>::store(a.b.grad_p, i, gpf);
@@ -1041,7 +965,7 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
         const float delta_f = c.delta[set] * dt * rho_i / c.refd[set];
         drhodt = drhodt + delta_f * lp;
         // BIe ElasticBounce.cl
-        if (bie && dt != 0.f) {
+        if (dt != 0.f) {
             float vh[3];
             for (int k = 0; k < D; k++)
                 vh[k] = uin[k] + hdt * acc[k];
@@ -1094,34 +1018,20 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
     float rin[4] = { 0.f, 0.f, 0.f, 0.f };
     Vec<D>::load(a.b.r_in, i, rin);
     float rn_[4] = { 0.f, 0.f, 0.f, 0.f }, un[4] = { 0.f, 0.f, 0.f, 0.f };
-    float rho_n;
-    if (c.scheme == AQUA_SCHEME_IMPROVED_EULER) {
-        // improved_euler.cl corrector: r_in, u_in, rho_in hold the sorted
-        // predictor output
-        const float DT = 0.5f * dt;
-        const float DT2 = DT * DT;
-        for (int k = 0; k < VS; k++) {
-            const float da = acc[k] - ain[k];
-            un[k] = uin[k] + DT * da;
-            rn_[k] = rin[k] + DT2 * da;
-        }
-        rho_n = a.b.rho_in[i] + DT * (drhodt - drhodt_in);
-    } else {
-        // midpoint relax
-        const float rl = c.relax_midpoint;
-        for (int k = 0; k < VS; k++)
-            acc[k] = rl * ain[k] + (1.f - rl) * acc[k];
-        drhodt = rl * drhodt_in + (1.f - rl) * drhodt;
-        // corrector
-        const float hdt2 = 0.5f * dt * dt;
-        for (int k = 0; k < VS; k++) {
-            rn_[k] = rin[k] + dt * uin[k] + hdt2 * acc[k];
-            un[k] = uin[k] + dt * acc[k];
-        }
-        rho_n = a.b.rho_in[i] + dt * drhodt;
+    // midpoint relax
+    const float rl = c.relax_midpoint;
+    for (int k = 0; k < VS; k++)
+        acc[k] = rl * ain[k] + (1.f - rl) * acc[k];
+    drhodt = rl * drhodt_in + (1.f - rl) * drhodt;
+    // corrector
+    const float hdt2 = 0.5f * dt * dt;
+    for (int k = 0; k < VS; k++) {
+        rn_[k] = rin[k] + dt * uin[k] + hdt2 * acc[k];
+        un[k] = uin[k] + dt * acc[k];
     }
+    const float rho_n = a.b.rho_in[i] + dt * drhodt;
     // BIe PST.cl
-    if (fluid && bie) {
+    if (fluid) {
         const float Ri = 0.5f * powf(T.m[i] / rho_n, 1.f / c.DIMS);
         for (int k = 0; k < NC; k++) {
             const uint32_t cn = neighbour_cell<D>(key_i, k, nx, nxy);
@@ -1164,10 +1074,9 @@ sweep_particle(const Consts& c, const StepArgs& a, uint32_t i, bool valid,
 
 // Persistent sweep: warps fetch cell-aligned chunks of <= 32 particles
 // NT threads per block, NQ queued neighbours per thread (power of 2, >= 64)
-// of type QE, candidate groups copied by the bulk-copy engine when BULK,
-// BI walls (cfd/BI.xml) when BI, else BIe walls
-template<int D, int NT, int NQ, typename QE, bool BULK, bool BI, int MODE,
-         int MINW = 20>
+// of type QE, candidate groups copied by the bulk-copy engine when BULK.
+// BIe walls, midpoint scheme (BI walls run the quad sweep)
+template<int D, int NT, int NQ, typename QE, bool BULK, int MODE, int MINW = 20>
 __global__ void __launch_bounds__(NT, MINW * 32 / NT)
 k_sweep(Consts c, StepArgs a)
 {
@@ -1213,7 +1122,7 @@ k_sweep(Consts c, StepArgs a)
                 break;
             const uint2 cw = a.b.chunks[ch];
             const bool valid = (uint32_t)lane < cw.y;
-            float v = sweep_particle<D, NT, NQ, QE, BULK, BI, MODE>(
+            float v = sweep_particle<D, NT, NQ, QE, BULK, MODE>(
                 c, a, valid ? cw.x + lane : cw.x, valid,
                 s_queue + (MODE == kSweepQueue ? threadIdx.x : 0),
                 s_cstart[warp], s_grp[warp], s_mbar[warp], phases,
@@ -1286,51 +1195,51 @@ launch_sweep_impl(const Consts& c, const StepArgs& a, unsigned grid,
         return cudaSuccess;
     switch (variant) {
     case 1:
-        k_sweep<D, 64, 128, uint16_t, false, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 128, uint16_t, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
         break;
     case 2:
-        k_sweep<D, 64, 64, uint32_t, false, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 64, uint32_t, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
         break;
     case 3:
-        k_sweep<D, 64, 128, uint16_t, true, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 128, uint16_t, true, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
         break;
     case 4:
-        k_sweep<D, 64, 64, uint32_t, true, false, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 64, uint32_t, true, kSweepQueue><<<grid, 64, 0, s>>>(c, a);
         break;
     case 5:
-        k_sweep<D, 64, 1, uint32_t, false, false, kSweepDirect><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 1, uint32_t, false, kSweepDirect><<<grid, 64, 0, s>>>(c, a);
         break;
     case 6:
-        k_sweep<D, 128, 1, uint32_t, false, false, kSweepDirect><<<grid, 128, 0, s>>>(c, a);
+        k_sweep<D, 128, 1, uint32_t, false, kSweepDirect><<<grid, 128, 0, s>>>(c, a);
         break;
     case 7:
-        k_sweep<D, 64, 1, uint32_t, true, false, kSweepDirect><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 1, uint32_t, true, kSweepDirect><<<grid, 64, 0, s>>>(c, a);
         break;
     case 8:
-        k_sweep<D, 128, 1, uint32_t, true, false, kSweepDirect><<<grid, 128, 0, s>>>(c, a);
+        k_sweep<D, 128, 1, uint32_t, true, kSweepDirect><<<grid, 128, 0, s>>>(c, a);
         break;
     // the same with the register budget of 28, 32 or 36 resident warps per
     // SM
     case 9:
-        k_sweep<D, 64, 1, uint32_t, true, false, kSweepDirect, 28><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 1, uint32_t, true, kSweepDirect, 28><<<grid, 64, 0, s>>>(c, a);
         break;
     case 10:
-        k_sweep<D, 128, 1, uint32_t, true, false, kSweepDirect, 28><<<grid, 128, 0, s>>>(c, a);
+        k_sweep<D, 128, 1, uint32_t, true, kSweepDirect, 28><<<grid, 128, 0, s>>>(c, a);
         break;
     case 11:
-        k_sweep<D, 64, 1, uint32_t, true, false, kSweepDirect, 32><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 1, uint32_t, true, kSweepDirect, 32><<<grid, 64, 0, s>>>(c, a);
         break;
     case 12:
-        k_sweep<D, 128, 1, uint32_t, true, false, kSweepDirect, 32><<<grid, 128, 0, s>>>(c, a);
+        k_sweep<D, 128, 1, uint32_t, true, kSweepDirect, 32><<<grid, 128, 0, s>>>(c, a);
         break;
     case 13:
-        k_sweep<D, 64, 1, uint32_t, true, false, kSweepDirect, 36><<<grid, 64, 0, s>>>(c, a);
+        k_sweep<D, 64, 1, uint32_t, true, kSweepDirect, 36><<<grid, 64, 0, s>>>(c, a);
         break;
     case 14:
-        k_sweep<D, 128, 1, uint32_t, true, false, kSweepDirect, 36><<<grid, 128, 0, s>>>(c, a);
+        k_sweep<D, 128, 1, uint32_t, true, kSweepDirect, 36><<<grid, 128, 0, s>>>(c, a);
         break;
     default:
-        k_sweep<D, 128, 128, uint16_t, false, false, kSweepQueue><<<grid, 128, 0, s>>>(c, a);
+        k_sweep<D, 128, 128, uint16_t, false, kSweepQueue><<<grid, 128, 0, s>>>(c, a);
         break;
     }
     return cudaGetLastError();

@@ -95,6 +95,9 @@ __constant__ uint8_t kHilbert2[64] = {
 // Where the step is swept by octant (sweep_by_octant()), a cell's clusters are
 // octants (8 consecutive places), joined while they fit into 8, if all of them do.
 constexpr int kClusterThreads = 256;
+// A cell of more particles (parked ones, no fluid cell: 512 with h = 4 spacings in
+// 3-D) would keep its warp for long: 20,000 parked particles in 2-D, 336 us a step.
+constexpr uint32_t kLargeCell = 1024;
 template<int D, bool CELLS>
 __global__ void __launch_bounds__(kClusterThreads)
 k_cell_clusters(Consts c, StepArgs a, const float4* pos)
@@ -104,10 +107,11 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
     constexpr uint32_t kWalls = 64, kProbes = 65, kNone = 66;
     __shared__ uint4 s_cell[kClusterThreads];  // (first, count, clusters before, -)
     __shared__ uint32_t s_cnt[NWARP][kNone];
-    __shared__ uint2 s_warp[NWARP];
+    __shared__ uint4 s_warp[NWARP];
+    __shared__ uint2 s_large[2];
     __shared__ uint32_t s_base;
-    // the curve (constant memory serves one address at a time: 216 us for 5.88M
-    // particles, now 150)
+    // the curve (constant memory serves one address at a time: 212 us for 5.88M
+    // particles, now 166)
     __shared__ uint8_t s_place[64];
     if (__syncthreads_or(threadIdx.x == 0 && a.sc->err))
         return;  // one read for the whole block
@@ -124,6 +128,34 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
             n = a.b.cells[key].y - s0;
     }
     const uint32_t P = a.cluster;  // 4 or 8
+    // CELLS = false: the block's part of a cell of more than kLargeCell
+    // particles, cut in sorted order
+    uint32_t large = 0;  // the particles from this position on, if a cluster starts here
+    if constexpr (!CELLS) {
+        if (threadIdx.x == 0) {
+            s_large[0] = s_large[1] = make_uint2(0u, 0u);
+            if (n == 0 && s0 < a.N) {
+                const uint2 se = a.b.cells[a.skeys[s0]];
+                if (se.y - se.x > kLargeCell)
+                    s_large[0] = se;
+            }
+        }
+        __syncthreads();
+        if (n > kLargeCell) {  // one at most
+            s_large[1] = make_uint2(s0, s0 + n);
+            n = 0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const uint2 se = s_large[k];
+            if (s0 >= se.x && s0 < se.y) {
+                a.b.cperm[s0] = s0;
+                large = (s0 - se.x) % P == 0 ? se.y - s0 : 0u;
+            }
+        }
+    }
+    const unsigned lb = __ballot_sync(0xffffffffu, large > 0);
     const uint32_t ncl = (n + P - 1u) / P;
     // exclusive scan over the block: cells and clusters
     uint32_t xc = ncl;
@@ -134,24 +166,31 @@ k_cell_clusters(Consts c, StepArgs a, const float4* pos)
             xc += y;
     }
     if (lane == 31)
-        s_warp[warp] = make_uint2((uint32_t)__popc(starts), xc);
+        s_warp[warp] = make_uint4((uint32_t)__popc(starts), xc, (uint32_t)__popc(lb), 0u);
     __syncthreads();
     uint32_t cells = 0, clusters = 0, n_cells = 0, n_clusters = 0;
+    uint32_t larges = 0, n_large = 0;
     for (int w = 0; w < NWARP; w++) {
-        const uint2 v = s_warp[w];
+        const uint4 v = s_warp[w];
         if (w < warp) {
             cells += v.x;
             clusters += v.y;
+            larges += v.z;
         }
         n_cells += v.x;
         n_clusters += v.y;
+        n_large += v.z;
     }
     if (n > 0)
         s_cell[cells + __popc(starts & lt)] = make_uint4(s0, n, clusters + xc - ncl, 0u);
     if (threadIdx.x == 0)
-        s_base = n_cells ? atomicAdd(&a.sc->n_chunks, CELLS ? n_cells : n_clusters) : 0u;
+        s_base = n_cells + n_large
+                     ? atomicAdd(&a.sc->n_chunks, CELLS ? n_cells : n_clusters + n_large)
+                     : 0u;
     __syncthreads();
     const uint32_t base = s_base;
+    if (large)
+        a.b.clu[base + n_clusters + larges + __popc(lb & lt)] = make_uint2(s0, min(P, large));
     for (uint32_t w = warp; w < n_cells; w += NWARP) {
         const uint4 cell = s_cell[w];
         const uint32_t first = cell.x, cnt = cell.y;
@@ -317,7 +356,7 @@ k_octants(Consts c, StepArgs a)
     const CaseScalars& cs = a.cs[a.dst.cid[s0]];
     const float scale = 4.f * c.idist;
     uint32_t n = 0;  // lane o < 8: particles of octant o along the curve
-    for (uint32_t b = se.x; b < se.y; b += 32) {
+    for (uint32_t b = se.y - se.x > kLargeCell ? se.y : se.x; b < se.y; b += 32) {
         uint32_t o = 8;
         if (b + lane < se.y && a.dst.imove[b + lane] > 0) {
             const float4 p = a.b.rec0[b + lane];

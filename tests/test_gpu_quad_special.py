@@ -65,3 +65,13 @@ def test_pairs_at_the_edge_of_the_support(dims, scale, seed):
     r[1:1 + len(g)] = g[:n - 1] * reach / 4
     c.r[:n, :dims] = r
     assert_same(c)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("n", [1023, 1025, 1500, 2200])
+def test_cells_of_very_many_particles(dims, n):
+    """One cell on both sides of the count from which its particles are cut into
+    clusters by position: starting within a block of positions and spanning
+    several."""
+    c = cloud(dims, n, 0.85, n + dims, 12)
+    assert_same(c)

@@ -185,8 +185,8 @@ struct StepBufs
     // ranges in `wcl` (first, end, case, clusters; the cell's clusters
     // start at index `first` of `clu`), the (first sorted index, count) of
     // the 9 rows of 3 cells around each in `crow`; clusters of <= 8
-    // particles of one cell octant as (first position in cperm, count);
-    // cperm = sorted indices in cluster order
+    // particles of one cell (k_cell_clusters; the quad sweep's too) as (first
+    // position in cperm, count); cperm = sorted indices in cluster order
     float4* rec0;
     float4* rec1;
     uint8_t* cell_mark;    // rate sample: cells around a probe (ncap)

@@ -867,13 +867,12 @@ static_assert(edge_mlp_smem<144>() <= 226 * 1024, "one CTA per SM");
 // columns; the epilogue multiplies by silu'(Zprev) and rounds to BF16.
 //
 // wgrad: dW += dY^T X and db += column sums of dY.  The reduction runs over
-// the M rows (edges or nodes), 128 per chunk: each chunk of dY and X is
-// staged transposed (dY^T: N rows of 128, padded with zero rows to the
-// MMA's 128; X^T: K rows of 128) into the K-major core-matrix layout, and
-// the MMAs accumulate over all the CTA's chunks in tensor memory.  One
-// extra row of ones in B makes the column K of the product the column sums
-// of dY (db).  At the end each CTA adds its partial dW, db to the outputs
-// with atomics.
+// the M rows (edges or nodes), 128 per chunk: each chunk of dY (padded with
+// zeros to the MMA's 128 outputs) and X is copied as its rows lie in memory,
+// both operands MN-major, and the MMAs accumulate over all the CTA's chunks in
+// tensor memory.  One extra output of ones in B makes the column K of the
+// product the column sums of dY (db).  At the end each CTA adds its partial
+// dW, db to the outputs with atomics.
 
 // bounded wait for a commit on `mbar` (phase parity `phase`); every thread
 // of the CTA returns the same verdict
@@ -1286,7 +1285,7 @@ aqua_gnn_edge_mlp_tc(uint32_t E, uint32_t K1, const uint16_t* X, uint32_t ldx,
     const aqua_status st = edge_mlp_configure(sms);
     if (st != AQUA_OK)
         return st;
-    // one CTA per SM (shared memory; 192 of the 512 TMEM columns)
+    // one CTA per SM (shared memory; it holds all 512 tensor-memory columns)
     const uint32_t tiles = (E + kTcRows - 1) / kTcRows;
     const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
     cudaStream_t s = (cudaStream_t)stream;

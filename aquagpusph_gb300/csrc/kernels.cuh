@@ -18,9 +18,9 @@ constexpr int kSortTile = kSortThreads * kSortItems;   // keys per block
 // prefetched by asynchronous copies: 7 = 64 threads, 8 = 128 threads;
 // those with the register budget of 28 resident warps per SM (9 = 64,
 // 10 = 128 threads), 32 (11, 12) or 36 (13, 14)
-// 15 to 17: the clustered sweep of the fast 3-D build (BIe walls, midpoint
-// scheme; 8 warps per block, 2,048 neighbour records staged per pass), the quad
-// sweep everywhere else
+// 15 to 17, alike: the clustered sweep of the fast 3-D build (BIe walls,
+// midpoint scheme; 8 warps per block, 2,048 neighbour records staged per pass),
+// the quad sweep everywhere else
 constexpr int kSweepClustered = 15;
 constexpr int kSweepVariants = 18;
 constexpr int kSweepClusteredDefault = 16;

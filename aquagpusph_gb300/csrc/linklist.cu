@@ -700,8 +700,11 @@ k_small_linklist(Consts c, const float* r, const int32_t* imove,
         sc->by_octant = 0;
         sc->by_cut = 0;
     }
-    // an error of an earlier step: the blocks read it before any of this
-    // launch's blocks can set it (rank 0, after the second cluster barrier)
+    // an error of an earlier step: the cluster's blocks read it before rank 0
+    // can set one (after the first cluster barrier).  The clusters that clear
+    // the cell table read it in no order with that: a table that an error of
+    // this step leaves partly cleared is read by no kernel, since all return on
+    // an error, and cleared by the first step after the error is reset.
     if (t == 0) {
         S.stop = sc->err;
         S.bad = 0;

@@ -43,7 +43,7 @@
 //
 // Instruction issue bounds both (72% of the slots, 24 warps an SM by shared
 // memory).  Off the lattice octants fill their clusters 5 to 7 of 8: 5.9M sheared
-// particles 9.39 ms a call, by box 8.2; 406,402: 1.09 ms, by box 0.79.  On a
+// particles 9.39 ms a call, by box 8.18; 406,402: 1.09 ms, by box 0.77.  On a
 // lattice at rest octants are perfect clusters and finding their neighbours takes
 // 1,365 instructions of a warp per cluster in place of 2,060: 5.88M particles 5.76
 // ms a step, by box 6.27.  Both in one kernel, chosen by cell, were 7 to 15% slower

@@ -900,7 +900,7 @@ k_sweep_cl(Consts c, StepArgs a)
                                 const float dy = fmaxf(fmaxf(lo[1] - r.y, r.y - hi[1]), 0.f);
                                 const float dz = fmaxf(fmaxf(lo[2] - r.z, r.z - hi[2]), 0.f);
                                 const bool in = dx * dx + dy * dy + dz * dz < R2;
-                                fl[v] = in && r.w > 0.f;
+                                fl[v] = in && !(r.w <= 0.f);  // a NaN is listed
                                 // the boundary elements matter to fluid only
                                 wa[v] = in && r.w < 0.f && any_fluid;
                                 bf[v] = __ballot_sync(0xffffffffu, fl[v]);

@@ -75,3 +75,31 @@ def test_cells_of_very_many_particles(dims, n):
     several."""
     c = cloud(dims, n, 0.85, n + dims, 12)
     assert_same(c)
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("n,spread", [(1, 0.2), (5, 0.5), (60, 0.9), (400, 1.9)])
+@pytest.mark.parametrize("name", ["rho", "m", "u"])
+def test_fast_sweeps_do_not_drop_a_nan(dims, n, spread, name):
+    """The default sweeps of the fast build: where the direct sweep's result is
+    NaN because a neighbour's value is, theirs is too."""
+    from aquagpusph_gb300.solver import Solver
+    c = cloud(dims, n, spread, 31 * n + dims, 8)
+    a = getattr(c, name)
+    a[(n // 2, 0) if a.ndim == 2 else n // 2] = np.nan
+    out = []
+    for variant, blocks in ((16, 3), (9, 14)):
+        sv = Solver(c.params, capacity=c.N)
+        sv.set_precision(True)
+        sv.set_tuning(variant, blocks)
+        sv.set_case(c)
+        sv.step(1, graph=True)
+        out.append(sv.get_case())
+        sv.close()
+    g, direct = out
+    fl = direct.imove == 1
+    for k in ("dudt", "drhodt", "rho", "shepard"):
+        x, y = np.asarray(getattr(g, k)), np.asarray(getattr(direct, k))
+        # the particle itself keeps a value that its own NaN does not reach
+        bad = fl.reshape((-1,) + (1,) * (x.ndim - 1)) & np.isnan(y) & ~np.isnan(x)
+        assert not bad.any(), k

@@ -103,3 +103,21 @@ def test_fast_sweeps_do_not_drop_a_nan(dims, n, spread, name):
         # the particle itself keeps a value that its own NaN does not reach
         bad = fl.reshape((-1,) + (1,) * (x.ndim - 1)) & np.isnan(y) & ~np.isnan(x)
         assert not bad.any(), k
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("name,value", [
+    ("m", np.nan), ("m", np.inf), ("m", -1.0), ("normal", np.nan), ("normal", np.inf),
+    ("u", np.inf), ("u", np.nan)])
+def test_boundary_elements_that_are_not_ordinary(dims, name, value):
+    """One boundary element with such an area, normal or velocity, among fluid
+    that lies within a radius of the wall, in and out of its support."""
+    c = cloud(dims, 240, 2.6, 5 + dims, 120)
+    h = c.params.h
+    c.r[:240:2, dims - 1] = np.float32(0.1 * h) * (1 + np.arange(120)) / 120
+    a = getattr(c, name)
+    if a.ndim == 2:
+        a[300, :dims] = value
+    else:
+        a[300] = value
+    assert_same(c)
